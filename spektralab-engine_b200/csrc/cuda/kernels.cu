@@ -866,10 +866,11 @@ __global__ void k_develop(const float* __restrict__ exposure, float* __restrict_
 // A pixel's nine Poisson draws take data-dependent paths: most PTRS draws end at the first attempt's
 // squeeze, the rest need the logarithm test, further attempts or (lam < 10) the product method. Run
 // per lane, a warp would wait on its slowest lane at every draw. Here each lane makes every draw's
-// first attempt in lockstep; a draw the squeeze does not settle goes to a ring of deferred draws in the
-// warp's shared memory, and whenever 32 are queued the whole warp finishes them, one per lane. Every
-// draw consumes the same uniforms in the same order and with the same arithmetic as spk_poisson, so the
-// counts are those of the per-lane sampler.
+// first attempt in lockstep, by approximations that settle it only where their error cannot matter
+// (squeeze_certain); every other draw goes to a ring in the warp's shared memory, from which the whole
+// warp takes 32 at a time, one attempt per lane, by the sampler's own operations (draw_attempt). Every
+// draw consumes the same uniforms in the same order as spk_poisson, so the counts are those of the
+// per-lane sampler.
 
 #ifndef SPKB_DEVELOP_WARPS
 #define SPKB_DEVELOP_WARPS 4
@@ -877,28 +878,12 @@ __global__ void k_develop(const float* __restrict__ exposure, float* __restrict_
 constexpr uint32_t kDrawWarps = SPKB_DEVELOP_WARPS;  // warps per block
 // resident blocks per SM the register allocation is held to (1: no cap)
 #ifndef SPKB_DEVELOP_MIN_BLOCKS
-#define SPKB_DEVELOP_MIN_BLOCKS 1
+#define SPKB_DEVELOP_MIN_BLOCKS 10
 #endif
-constexpr uint32_t kDrawRing = 64;  // holds the < 32 left over plus one draw's 32
-
-struct DeferredDraw {
-    float lam, b, a, vr;        // the squeeze's PTRS constants (kinds 1, 2); lam alone for kind 0
-    float loglam, loginvalpha;  // the full test's constants, once formed (kTagInited)
-    float V, k, us;             // the last attempt's full test, pending (kind 1)
-    uint32_t w2, w3;            // words z, w of the last Philox block: the next attempt's uniforms when it is odd
-    uint32_t tag;               // kind | kTagInited | stream << 3 | slot << 11 | next attempt << 20
-};
-// kinds: 0 product method (lam < 10 or NaN); 1 the last attempt needs the full test; 2 it was rejected.
-// slot = draw * 32 + lane: the draw's pixel is the warp's first plus the lane.
-constexpr uint32_t kResStride = kDrawWarps * 32;  // a draw's row in the block's lambda / result array
-constexpr uint32_t kTagInited = 4u;
-__device__ __forceinline__ uint32_t draw_tag(uint32_t kind, uint32_t stream, uint32_t slot, uint32_t next) {
-    return kind | (stream << 3) | (slot << 11) | (next << 20);
-}
 
 // log(k!) for k = 0 .. kLgammaTable - 1, each the sampler's own spk_lgamma_k(k + 1) computed by this
 // device once per process (k_lgamma_table): the full test's largest single cost, a table read instead.
-constexpr uint32_t kLgammaTable = 4096;
+constexpr uint32_t kLgammaTable = 65536;
 __device__ float g_lgamma[kLgammaTable];
 
 __global__ void k_lgamma_table() {
@@ -915,190 +900,314 @@ __device__ __forceinline__ int ptrs_test_table(const spk_ptrs* p, float V, float
     return L <= Rt;
 }
 
-// One step of a deferred draw, exactly as spk_ptrs_from runs it: the last attempt's pending full test
-// (kind 1), then, unless that accepted, the next attempt's uniforms and squeeze. Returns true once the
-// draw's count is in res; false with e holding the state to queue again (kind 1 or 2, the next attempt).
-// A product-method draw (kind 0) ends in one step. The test's constants (log lam, log 1 / alpha) are
-// formed the first time a draw reaches the test and travel with it. pixel0: the warp's first pixel; res:
-// the warp's results, draw k of lane j at res[k * kResStride + j].
-__device__ __forceinline__ bool finish_step(DeferredDraw& e, uint32_t seed, uint32_t pixel0, float* res_warp) {
-    const uint32_t kind = e.tag & 3u, stream = (e.tag >> 3) & 0xFFu, slot = (e.tag >> 11) & 0x1FFu;
-    const uint32_t it = e.tag >> 20;
-    const uint32_t pixel = pixel0 + (slot & 31u);
-    float* res = res_warp + (slot >> 5) * kResStride + (slot & 31u);
-    if (kind == 0u) {
-        spk_stream g;
-        spk_stream_init(&g, pixel, stream, seed);
-        *res = spk_poisson_product(e.lam, &g);
+// PTX approximations: sqrt and reciprocal within 2^-23 relative; log2 within 2^-22, relative outside [1/2, 2]
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float log2_approx(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// The sampler's full test (ptrs_test_table) with its left side, log V + log(1 / alpha) - log(a / us^2 + b),
+// taken as one approximate logarithm. The right side's rounding reaches far above that, so it is formed by
+// the sampler's own operations. The approximate left side lies within 4e-5 of the sampler's (its binary32
+// logarithms up to 37 in magnitude: at most 2e-5; lg2.approx: at most 1.4e-5; the argument's rounding
+// 1e-6): a test decided by more than 1e-4 stands, any other (about 2 in 10,000) runs the sampler's.
+__device__ __forceinline__ bool ptrs_accepts(spk_ptrs* p, float V, float k, float us) {
+    const float lg = k < float(kLgammaTable) ? g_lgamma[int(k)] : spk_lgamma_k(SPK_ADD(k, 1.0f));
+    p->loglam = spk_logf_normal(p->lam, 0);
+    const float Rt = SPK_SUB(SPK_ADD(-p->lam, SPK_MUL(k, p->loglam)), lg);
+    const float us2 = us * us, b34 = p->b - 3.4f;
+    const float num = (V * us2) * fmaf(1.1239f, b34, 1.1328f), den = b34 * fmaf(p->b, us2, p->a);
+    const float L = 0.693147181f * log2_approx(num * rcp_approx(den));
+    if (fabsf(L - Rt) > 1e-4f) return L <= Rt;
+    spk_ptrs_init_test(p);
+    return ptrs_test_table(p, V, k, us);
+}
+
+// Draws whose first attempt the lockstep below does not settle are queued as one word each: slot (draw *
+// 32 + lane) | attempt << 9.
+constexpr uint32_t kDrawRing = 512;  // at most the warp's 288 draws are queued at a time
+
+// Attempt `it` of a queued draw of lambda lm >= 10, exactly as spk_ptrs_from runs it (the squeeze, then the
+// full test). The count replaces the lambda in *res; false when the attempt was rejected.
+__device__ __forceinline__ bool draw_attempt(float* res, float lm, uint32_t pixel, uint32_t stream, uint32_t seed,
+                                             uint32_t it) {
+    if (it == 64u) {
+        *res = SPK_FLOOR(lm);
         return true;
     }
     spk_ptrs p;
-    p.lam = e.lam;
-    p.b = e.b;
-    p.a = e.a;
-    p.vr = e.vr;
-    bool inited = (e.tag & kTagInited) != 0u;
-    if (kind == 1u) {
-        if (inited) {
-            p.loglam = e.loglam;
-            p.loginvalpha = e.loginvalpha;
-        } else {
-            spk_ptrs_init_test(&p);
-            e.loglam = p.loglam;
-            e.loginvalpha = p.loginvalpha;
-            inited = true;
-        }
-        if (ptrs_test_table(&p, e.V, e.k, e.us)) {
-            *res = e.k;
-            return true;
-        }
+    spk_ptrs_init(&p, lm);
+    // uniforms 2 it and 2 it + 1: words x, y (it even) or z, w (it odd) of Philox block it / 2
+    spk_u4 c4;
+    c4.x = pixel;
+    c4.y = stream;
+    c4.z = it >> 1;
+    c4.w = 0u;
+    const spk_u4 b = spk_philox(c4, seed, 0u);
+    const bool odd = (it & 1u) != 0u;
+    const float V = spk_uniform(odd ? b.w : b.y);
+    float k, us;
+    const int r = spk_ptrs_squeeze(&p, spk_uniform(odd ? b.z : b.x), V, &k, &us);
+    if (r == SPK_PTRS_REJECT || (r == SPK_PTRS_TEST && !ptrs_accepts(&p, V, k, us))) return false;
+    *res = k;
+    return true;
+}
+
+// The rounds of a pixel's first Philox block (counter (pixel, stream, 0, 0), key (seed, 0)) that do not
+// depend on the stream, shared by its nine draws: the second round's (x, y) and the third round's first
+// product, with the round keys and the words they meet folded in.
+struct PhiloxHead {
+    uint32_t y3k;       // y of round 2 ^ k0 of round 3
+    uint32_t z2;        // lo(M0 pixel) ^ k1 of round 2: z of round 2 is this ^ hi(M0 (stream ^ seed))
+    uint32_t z3k, w3;   // hi(M0 x2) ^ k1 of round 3, lo(M0 x2)
+};
+__device__ __forceinline__ PhiloxHead philox_head(uint32_t pixel, uint32_t seed) {
+    const uint64_t p0 = uint64_t(SPK_PHILOX_M0) * pixel;
+    const uint64_t p1 = uint64_t(SPK_PHILOX_M1) * uint32_t(p0 >> 32);
+    const uint64_t p3 = uint64_t(SPK_PHILOX_M0) * (uint32_t(p1 >> 32) ^ (seed + SPK_PHILOX_W0));
+    PhiloxHead h;
+    h.y3k = uint32_t(p1) ^ (seed + 2u * SPK_PHILOX_W0);
+    h.z2 = uint32_t(p0) ^ SPK_PHILOX_W1;
+    h.z3k = uint32_t(p3 >> 32) ^ (2u * SPK_PHILOX_W1);
+    h.w3 = uint32_t(p3);
+    return h;
+}
+// the block's words; sh, sl: the halves of M0 (stream ^ seed)
+__device__ __forceinline__ spk_u4 philox_first(const PhiloxHead& h, uint32_t sh, uint32_t sl, uint32_t seed) {
+    const uint64_t p1 = uint64_t(SPK_PHILOX_M1) * (sh ^ h.z2);
+    spk_u4 c;
+    c.x = uint32_t(p1 >> 32) ^ h.y3k;
+    c.y = uint32_t(p1);
+    c.z = h.z3k ^ sl;
+    c.w = h.w3;
+#pragma unroll
+    for (uint32_t r = 3; r < 10; ++r) {
+        const uint64_t a = uint64_t(SPK_PHILOX_M0) * c.x, b = uint64_t(SPK_PHILOX_M1) * c.z;
+        c.x = uint32_t(b >> 32) ^ c.y ^ (seed + r * SPK_PHILOX_W0);
+        c.y = uint32_t(b);
+        c.z = uint32_t(a >> 32) ^ c.w ^ (r * SPK_PHILOX_W1);
+        c.w = uint32_t(a);
     }
-    if (it == 64u) {
-        *res = SPK_FLOOR(p.lam);
-        return true;
+    return c;
+}
+
+// Four more uniforms of the product method: prod times each in turn, and how many products stayed above
+// E = exp(-lambda) (they never rise, so these come first); the draw is done once one has not
+__device__ __forceinline__ uint32_t product_block(const spk_u4& words, float E, float& prod) {
+    const uint32_t wd[4] = {words.x, words.y, words.z, words.w};
+    uint32_t above = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        prod = SPK_MUL(prod, spk_uniform(wd[i]));
+        above += prod > E ? 1u : 0u;
     }
-    // attempt it takes uniforms 2 it and 2 it + 1: words x, y of Philox block it / 2 (it even, keeping z, w
-    // for attempt it + 1) or the kept z, w (it odd)
-    uint32_t wu = e.w2, wv = e.w3;
-    if ((it & 1u) == 0u) {
+    return above;
+}
+
+// spk_poisson_product, a Philox block (four uniforms) per turn
+__device__ __forceinline__ float poisson_product(float lam, uint32_t pixel, uint32_t stream, uint32_t seed) {
+    const float E = spk_expf(-lam);
+    float prod = 1.0f;
+    uint32_t n = 0;
+#pragma unroll 1
+    for (uint32_t j = 0; j < 128u; ++j) {
         spk_u4 c4;
         c4.x = pixel;
         c4.y = stream;
-        c4.z = it >> 1;
+        c4.z = j;
         c4.w = 0u;
-        const spk_u4 b = spk_philox(c4, seed, 0u);
-        wu = b.x;
-        wv = b.y;
-        e.w2 = b.z;
-        e.w3 = b.w;
+        const uint32_t above = product_block(spk_philox(c4, seed, 0u), E, prod);
+        n += above;
+        if (above < 4u) break;
     }
-    const float V = spk_uniform(wv);
-    float k, us;
-    const int r = spk_ptrs_squeeze(&p, spk_uniform(wu), V, &k, &us);
-    if (r == SPK_PTRS_ACCEPT) {
-        *res = k;
-        return true;
-    }
-    e.V = V;
-    e.k = k;
-    e.us = us;
-    e.tag = draw_tag(r == SPK_PTRS_TEST ? 1u : 2u, stream, slot, it + 1u) | (inited ? kTagInited : 0u);
-    return false;
+    return float(n);
 }
 
+// A first attempt (uniform words wu, wv) that the sampler's squeeze accepts beyond doubt: true, and k the
+// sampler's count. The squeeze is evaluated with approximate square root and reciprocals; it stands when
+// V lies more than 1e-6 below v_r and the count's argument lies further from an integer than both
+// evaluations' errors: 2 ulp of the argument (below lam + 0.74 b) for the last sums, and 8e-7 relative of
+// (2 a / us + b) |U| < 0.74 b before them. U, us and V are the sampler's own values.
+__device__ __forceinline__ bool squeeze_certain(float lam, uint32_t wu, uint32_t wv, float& k) {
+    const float U = __fmaf_rn(__fadd_rn(float(wu >> 8), 0.5f), 5.9604644775390625e-08f, -0.5f);
+    const float us = __fsub_rn(0.5f, fabsf(U));
+    const float V = spk_uniform(wv);
+    const float b = fmaf(2.53f, sqrt_approx(lam), 0.931f);
+    const float vr = fmaf(-3.6224f, rcp_approx(b - 2.0f), 0.9277f - 1e-6f);
+    const float g = fmaf(fmaf(fmaf(0.04966f, b, -0.118f), rcp_approx(us), b), U, lam + 0.43f);
+    k = floorf(g);
+    const float frac = g - k, tol = fmaf(lam, 4e-7f, 1.5e-6f * b);
+    return lam >= 10.0f && us >= 0.07f && V <= vr && frac >= tol && frac <= 1.0f - tol;
+}
+
+// curve_lookup and layer_densities on the packed tables (DevelopArgs::packed): the same interval and the
+// same operations, the interval's values read with one vector load, the ends by clamping onto the first or
+// last entry. A NaN stays one. The densities' axis is the film's own curve, far from evenly spaced: its
+// bisection took ten dependent loads, the guide's bucket leaves none to four.
+__device__ __forceinline__ float curve_packed(const DevelopArgs& q, uint32_t c, float v) {
+    const float4* e = reinterpret_cast<const float4*>(q.curve4) + size_t(c) * q.K;
+    v = v < q.cgrid.x0 ? q.cgrid.x0 : v;
+    v = v > q.curve_last ? q.curve_last : v;
+    const int j = min(max(int((v - q.cgrid.x0) * q.cgrid.s), 0), int(q.K) - 2);
+    float4 t = __ldg(e + j);
+    const float next = __ldg(&e[j + 1].x);
+    if (t.x > v) t = __ldg(e + j - 1);
+    else if (next <= v) t = __ldg(e + j + 1);
+    return t.z + ((v - t.x) * t.y) * t.w;
+}
+__device__ __forceinline__ void layers_packed(const DevelopArgs& q, uint32_t c, float v, float dl[3]) {
+    const float* e = q.layer8 + size_t(c) * q.gK * 8;
+    v = v < q.guide_x0[c] ? q.guide_x0[c] : v;
+    v = v > q.axis_last[c] ? q.axis_last[c] : v;
+    const uint32_t g = __ldg(q.guide + c * kGuide + min(uint32_t(max(int((v - q.guide_x0[c]) * q.guide_s[c]), 0)), kGuide - 1u));
+    uint32_t j = g & 0xFFFFu, hi = g >> 16;
+    while (j < hi) {
+        const uint32_t mid = (j + hi + 1u) / 2u;
+        if (__ldg(e + 8 * mid) <= v) j = mid;
+        else hi = mid - 1u;
+    }
+    float t[8];
+    ld32(e + 8 * j, t);
+    const float f = (v - t[0]) * t[1];
+#pragma unroll
+    for (int l = 0; l < 3; ++l) dl[l] = t[2 + 2 * l] + f * t[3 + 2 * l];
+}
+
+// spk_sublayer_lambda with the quotients by a constant's reciprocal (exact after its remainder's
+// correction: Brisebarre, Muller and Raina, "Accelerating correctly rounded floating-point division when
+// the divisor is known in advance", IEEE Trans. Computers 53 (2004)) and by spk_div_normal
+__device__ __forceinline__ float sublayer_lambda_fast(float d, float D, float rD, float n, float u, float* sat_out) {
+    const float q0 = __fmul_rn(d, rD);
+    float q = __fmaf_rn(__fmaf_rn(-q0, D, d), rD, q0);
+    q = q < 1e-6f ? 1e-6f : (q > 0.999999f ? 0.999999f : q);
+    const float sat = SPK_SUB(1.0f, SPK_MUL(SPK_MUL(q, u), 0.999999f));
+    *sat_out = sat;
+    return SPK_MUL(SPK_DIV_NORMAL(n, sat), q);
+}
+
+// PRODUCT: a warp with a draw of lambda below this runs the product method's first four uniforms in
+// lockstep (at 4, 6, 8 and 10 the 24-megapixel export measured the same within 0.5 %).
+constexpr float kProductLockstep = 6.0f;
+
+// One pixel per lane. Every lane makes the first attempt of its nine draws, straight-line code with no
+// branch; a draw that squeeze_certain does not settle (26 % in the 4K benchmark frame) is queued in the
+// warp's ring as its slot alone, and the warp then takes 32 queued draws at a time, one attempt each, the
+// rejected queued again behind the rest; product-method draws (lambda < 10, or NaN) are set aside and run
+// last, so that a warp runs one method at a time. The kernel is bound by instruction issue (73 % of the
+// slots, 84 warp instructions a pixel): 4K benchmark frame 1.48 ms with ten-step bisections of the
+// densities' axis, general divides and the whole PTRS state in the ring, 0.83 this way.
+// Ten blocks per SM: 0.826 ms against 0.840 (nine), 0.865 (no cap); eleven slow the exports by 2 %.
+template <bool PACKED, bool PRODUCT>
 __global__ void __launch_bounds__(kDrawWarps * 32, SPKB_DEVELOP_MIN_BLOCKS) k_develop_layers(const float* __restrict__ exposure,
                                                                     float* __restrict__ out, uint32_t w,
                                                                     uint32_t blocks_per_row,
                                                                     const __grid_constant__ DevelopArgs q) {
-    __shared__ DeferredDraw ring[kDrawWarps][kDrawRing];
-    __shared__ float lam[9][kDrawWarps * 32], scale[9][kDrawWarps * 32];  // [c * 3 + l][thread]
+    __shared__ uint16_t ring[kDrawWarps][kDrawRing], product_list[kDrawWarps][9 * 32];
+    __shared__ float lam[kDrawWarps][9 * 32], scale[9][kDrawWarps * 32];  // [c * 3 + l]; a count replaces its lambda
     const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5, tid = threadIdx.x;
     const uint32_t y = blockIdx.x / blocks_per_row;
     const uint32_t x = (blockIdx.x - y * blocks_per_row) * (kDrawWarps * 32) + threadIdx.x;
     const bool live = x < w;
     const uint32_t pixel = y * q.width + x;
     const size_t o = 3 * (size_t(y) * w + x);
-
-    // lambda and the count's scale of the nine draws, [c][l], kept in shared memory
+    uint16_t* ringw = ring[wi];
+    uint16_t* productw = product_list[wi];
+    float* resw = lam[wi];
+    const uint32_t below = (1u << lane) - 1u;
+    const PhiloxHead head0 = philox_head(pixel, q.seed);
+    uint32_t tail = 0;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
+    for (uint32_t c = 0; c < 3; ++c) {
         float dl[3] = {0.0f, 0.0f, 0.0f};
         if (live) {
             float L = log10f(fmaxf(exposure[o + c], 0.0f) + 1e-10f);
             if (q.chi) L = __fsub_rn(L, q.chi[o + c]);  // DIR couplers: the corrected log exposure, the y0 curve
-            const float D = curve_lookup(q.cx, q.cinv, q.cy + size_t(c) * q.K, q.K, q.cgrid, L);
-            layer_densities(q, uint32_t(c), q.positive ? -D : D, dl);
+            if (PACKED) {
+                const float D = curve_packed(q, c, L);
+                layers_packed(q, c, q.positive ? -D : D, dl);
+            } else {
+                const float D = curve_lookup(q.cx, q.cinv, q.cy + size_t(c) * q.K, q.K, q.cgrid, L);
+                layer_densities(q, c, q.positive ? -D : D, dl);
+            }
         }
 #pragma unroll
-        for (int l = 0; l < 3; ++l) {
-            const int lc = l * 3 + c;
-            float sat = 1.0f;
-            lam[c * 3 + l][tid] =
-                live ? spk_sublayer_lambda(dl[l] + q.dmin_l[lc], q.sat_d[lc], q.count[lc], q.uniformity[c], &sat)
-                     : 0.0f;
-            if (q.lam_out && live) q.lam_out[size_t(pixel) * 9 + c * 3 + l] = lam[c * 3 + l][tid];
-            scale[c * 3 + l][tid] = SPK_MUL(q.unit[lc], sat);  // unit: SPK_DIV(sat_d, count), formed once
-        }
-    }
-
-    DeferredDraw* ringw = ring[wi];
-    // a draw's count replaces its lambda once the lockstep has read it: lam[k][tid] holds draw k of thread
-    // tid until its attempt 0, then its count
-    float* resw = &lam[0][wi * 32u];
-    uint32_t head = 0, tail = 0;
-#pragma unroll 1
-    for (uint32_t k = 0; k < 9u; ++k) {
-        const uint32_t stream = SPK_STREAM_GRAIN(k / 3u, k % 3u);
-        bool defer = false;
-        float value = 0.0f;
-        DeferredDraw d{};
-        uint32_t kind = 0u;
-        const float lm = lam[k][tid];
-        d.lam = lm;
-        if (live) {
-            if (lm >= 10.0f) {
-                spk_ptrs p;
-                spk_ptrs_init(&p, lm);
-                spk_u4 c4;
-                c4.x = pixel;
-                c4.y = stream;
-                c4.z = 0u;
-                c4.w = 0u;
-                const spk_u4 b0 = spk_philox(c4, q.seed, 0u);
-                float kk, us;
-                const int r = spk_ptrs_squeeze(&p, spk_uniform(b0.x), spk_uniform(b0.y), &kk, &us);
-                if (r == SPK_PTRS_ACCEPT) {
-                    value = kk;
-                } else {
-                    defer = true;
-                    kind = r == SPK_PTRS_TEST ? 1u : 2u;
-                    d.b = p.b;
-                    d.a = p.a;
-                    d.vr = p.vr;
-                    d.V = spk_uniform(b0.y);
-                    d.k = kk;
-                    d.us = us;
-                    d.w2 = b0.z;
-                    d.w3 = b0.w;
+        for (uint32_t l = 0; l < 3; ++l) {
+            const uint32_t lc = l * 3 + c, k = c * 3 + l;
+            float sat = 1.0f, value;
+            const float d = dl[l] + q.dmin_l[lc];
+            const float lm =
+                PACKED ? sublayer_lambda_fast(d, q.sat_d[lc], q.rcp_sat_d[lc], q.count[lc], q.uniformity[c], &sat)
+                       : spk_sublayer_lambda(d, q.sat_d[lc], q.count[lc], q.uniformity[c], &sat);
+            if (q.lam_out && live) q.lam_out[size_t(pixel) * 9 + k] = lm;
+            scale[k][tid] = SPK_MUL(q.unit[lc], sat);  // unit: SPK_DIV(sat_d, count), formed once
+            const spk_u4 words = philox_first(head0, q.stream_hi[k], q.stream_lo[k], q.seed);
+            bool settled = squeeze_certain(lm, words.x, words.y, value);
+            // the product method's first four uniforms, where some lane's draw is likely to end with them
+            if (PRODUCT && __any_sync(0xFFFFFFFFu, lm < kProductLockstep)) {
+                float prod = 1.0f;
+                const uint32_t above = product_block(words, spk_expf_normal(-fminf(lm, 80.0f)), prod);
+                if (lm < 10.0f && above < 4u) {
+                    value = float(above);
+                    settled = true;
                 }
-            } else {
-                defer = true;
             }
-        }
-        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, defer);
-        if (defer) {
-            d.tag = draw_tag(kind, stream, k * 32u + lane, 1u);
-            ringw[(tail + __popc(mask & ((1u << lane) - 1u))) & (kDrawRing - 1u)] = d;
-        } else {
-            resw[k * kResStride + lane] = value;
-        }
-        tail += __popc(mask);
-        // one step for 32 deferred draws at a time, the unfinished queued again behind the rest; after the
-        // last draw, until none is left. The ring holds at most 63: fewer than 32 left over plus 32 queued.
-        while (tail - head >= 32u || (k == 8u && tail != head)) {
-            __syncwarp();
-            const uint32_t n = min(tail - head, 32u);
-            DeferredDraw e;
-            bool again = false;
-            if (lane < n) {
-                e = ringw[(head + lane) & (kDrawRing - 1u)];
-                again = !finish_step(e, q.seed, pixel - lane, resw);
-            }
-            head += n;
-            __syncwarp();
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, again);
-            if (again) ringw[(tail + __popc(m & ((1u << lane) - 1u))) & (kDrawRing - 1u)] = e;
-            tail += __popc(m);
-            __syncwarp();
+            resw[k * 32u + lane] = settled ? value : lm;
+            const uint32_t open = __ballot_sync(0xFFFFFFFFu, live && !settled);
+            if (live && !settled) ringw[tail + __popc(open & below)] = uint16_t(k * 32u + lane);
+            tail += __popc(open);
         }
     }
+    __syncwarp();
+    const auto stream_of = [](uint32_t slot) {
+        const uint32_t k = slot >> 5, c = k / 3u;
+        return SPK_STREAM_GRAIN(c, k - 3u * c);
+    };
+    const uint32_t pixel0 = pixel - lane;
+    uint32_t n_product = 0;
+    for (uint32_t head = 0; tail != head;) {
+        const uint32_t n = min(tail - head, 32u);
+        uint32_t slot = 0, it = 0;
+        bool again = false, product = false;
+        if (lane < n) {
+            const uint32_t e = ringw[(head + lane) & (kDrawRing - 1u)];
+            slot = e & 511u;
+            it = e >> 9;
+            const float lm = resw[slot];
+            product = !(lm >= 10.0f);
+            if (!product) again = !draw_attempt(resw + slot, lm, pixel0 + (slot & 31u), stream_of(slot), q.seed, it);
+        }
+        head += n;
+        __syncwarp();
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, again), mp = __ballot_sync(0xFFFFFFFFu, product);
+        if (again) ringw[(tail + __popc(m & below)) & (kDrawRing - 1u)] = uint16_t(slot | (it + 1u) << 9);
+        if (product) productw[n_product + __popc(mp & below)] = uint16_t(slot);
+        tail += __popc(m);
+        n_product += __popc(mp);
+        __syncwarp();
+    }
+    for (uint32_t i = lane; i < n_product; i += 32u) {
+        const uint32_t slot = productw[i];
+        resw[slot] = poisson_product(resw[slot], pixel0 + (slot & 31u), stream_of(slot), q.seed);
+    }
+    __syncwarp();
     if (!live) return;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         float val[3];
 #pragma unroll
         for (int l = 0; l < 3; ++l) {
-            const float cnt = resw[(c * 3 + l) * kResStride + lane];
+            const float cnt = resw[(c * 3 + l) * 32 + lane];
             if (q.counts_out) q.counts_out[size_t(pixel) * 9 + c * 3 + l] = cnt;
             val[l] = SPK_MUL(cnt, scale[c * 3 + l][tid]);
         }
@@ -1381,7 +1490,18 @@ void develop(const float* exposure, float* out, const DevelopArgs& a, uint32_t w
         develop_prepare(s);
         const uint32_t bx = div_up(w, kDrawWarps * 32);
         Probe p("develop_layers", s);
-        k_develop_layers<<<bx * h, kDrawWarps * 32, 0, s>>>(exposure, out, w, bx, a);
+        // The product method's lockstep pays where many lambdas are below 6: with DIR couplers, whose
+        // corrected densities reach far down, and pixels small against a grain. Measured with couplers at
+        // 1920 x 1280, without and with it: 52 um (2,800 grains a pixel) 0.28 / 0.31 ms, 18 um (340) 0.38 / 0.41,
+        // 12.5 um (160) 0.42 / 0.43 on a photograph and 0.51 / 0.50 on noise, 7.8 um (63) 0.41 / 0.37, 5.7 um
+        // (34) 0.38 / 0.32; without couplers it never gained more than 2 %.
+        float mean = 0.0f;
+        for (int i = 0; i < 9; ++i) mean += a.count[i] / 9.0f;
+        const bool product = a.chi && mean < 160.0f;
+        const dim3 g(bx * h), b(kDrawWarps * 32);
+        if (!a.packed) k_develop_layers<false, true><<<g, b, 0, s>>>(exposure, out, w, bx, a);
+        else if (product) k_develop_layers<true, true><<<g, b, 0, s>>>(exposure, out, w, bx, a);
+        else k_develop_layers<true, false><<<g, b, 0, s>>>(exposure, out, w, bx, a);
         return;
     }
     const dim3 b(32, 4), g(div_up(w, 32), div_up(h, 4));

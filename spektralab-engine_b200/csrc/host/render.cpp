@@ -8,6 +8,7 @@
 #include "../cuda/iir.hpp"
 #include "../cuda/launch.hpp"
 #include "../cuda/vjp.hpp"
+#include "../grain_sampler.h"
 #include "blur_plan.h"
 #include "status.hpp"
 #include "tiers.hpp"
@@ -19,6 +20,33 @@ namespace {
 void upload(Pool& pool, cudaStream_t s, DevBuffer& dst, const void* src, size_t bytes) {
     dst = pool.persistent(bytes);
     cuda_check(cudaMemcpyAsync(dst.ptr(), src, bytes, cudaMemcpyHostToDevice, s), "table upload");
+}
+
+// The bucket of value v on an axis from x0: the binary32 operations of the develop kernel.
+float guide_scale(float x0, float last) { return f32(double(kGuide) / (double(last) - double(x0))); }
+uint32_t guide_bucket(float v, float x0, float s) {
+    const float t = (v - x0) * s;
+    return t >= float(kGuide) ? kGuide - 1 : uint32_t(t);
+}
+// The guide needs an axis that never falls, from a first point below the second (a value at the first
+// point then lies in interval 0), short enough for its 16-bit intervals.
+bool guide_fits(const float* x, uint32_t K, uint32_t stride) {
+    if (K < 2 || K > 65535 || !(x[stride] > x[0])) return false;
+    for (uint32_t j = 0; j + 1 < K; ++j)
+        if (!(x[size_t(j + 1) * stride] >= x[size_t(j) * stride])) return false;
+    const float s = guide_scale(x[0], x[size_t(K - 1) * stride]);
+    return std::isfinite(s) && s > 0.0f;
+}
+// The bucket of a value rises with it, so the interval of a value in bucket b is at least the last point
+// whose bucket is below b and at most the last whose bucket is b.
+void fill_guide(const float* x, uint32_t K, uint32_t stride, uint32_t* guide) {
+    const float x0 = x[0], s = guide_scale(x0, x[size_t(K - 1) * stride]);
+    uint32_t j = 0;  // points in the buckets below b
+    for (uint32_t b = 0; b < kGuide; ++b) {
+        const uint32_t first = j == 0 ? 0 : j - 1;
+        while (j < K && guide_bucket(x[size_t(j) * stride], x0, s) <= b) ++j;
+        guide[b] = first | (j == 0 ? 0u : j - 1) << 16;
+    }
 }
 
 }  // namespace
@@ -48,16 +76,49 @@ void upload_tables(Pool& pool, cudaStream_t s, Pipeline& p) {
             }
         upload(pool, s, p.dev.patches, pt.data(), pt.size() * sizeof(float));
     }
-    std::vector<float> c(8 * size_t(f.K));
-    std::memcpy(c.data(), f.cx.data(), f.K * sizeof(float));
-    std::memcpy(c.data() + f.K, f.cinv.data(), f.K * sizeof(float));
-    std::memcpy(c.data() + 2 * f.K, f.cy.data(), 3 * f.K * sizeof(float));
-    std::memcpy(c.data() + 5 * f.K, f.cy0.data(), 3 * f.K * sizeof(float));
+    const size_t K = f.K;
+    std::vector<float> c(32 * K);
+    std::memcpy(c.data(), f.cx.data(), K * sizeof(float));
+    std::memcpy(c.data() + K, f.cinv.data(), K * sizeof(float));
+    std::memcpy(c.data() + 2 * K, f.cy.data(), 3 * K * sizeof(float));
+    std::memcpy(c.data() + 5 * K, f.cy0.data(), 3 * K * sizeof(float));
+    for (size_t t = 0; t < 6; ++t)  // y of the three channels, then y0
+        for (size_t k = 0; k < K; ++k) {
+            const float* y = c.data() + (2 + t) * K;
+            const bool end = k + 1 == K;
+            float* o = c.data() + 8 * K + (t * K + k) * 4;
+            o[0] = f.cx[k];
+            o[1] = end ? 0.0f : f.cinv[k];
+            o[2] = y[k];
+            o[3] = end ? 0.0f : y[k + 1] - y[k];
+        }
     upload(pool, s, p.dev.curves, c.data(), c.size() * sizeof(float));
     if (f.grain && f.grain->K) {
-        upload(pool, s, p.dev.gaxis, f.grain->axis.data(), f.grain->axis.size() * sizeof(float));
-        upload(pool, s, p.dev.ginv, f.grain->inv.data(), f.grain->inv.size() * sizeof(float));
-        upload(pool, s, p.dev.glayers, f.grain->layers.data(), f.grain->layers.size() * sizeof(float));
+        const GrainSetup& g = *f.grain;
+        const size_t gK = g.K;
+        std::vector<float> t(39 * gK + 3 * kGuide);
+        for (size_t ch = 0; ch < 3; ++ch)
+            for (size_t k = 0; k < gK; ++k) {
+                const bool end = k + 1 == gK;
+                float* o = t.data() + (ch * gK + k) * 8;
+                o[0] = g.axis[3 * k + ch];
+                o[1] = end ? 0.0f : g.inv[3 * k + ch];
+                for (size_t l = 0; l < 3; ++l) {
+                    const float y = g.layers[(k * 3 + l) * 3 + ch];
+                    o[2 + 2 * l] = y;
+                    o[3 + 2 * l] = end ? 0.0f : g.layers[((k + 1) * 3 + l) * 3 + ch] - y;
+                }
+            }
+        std::copy(g.axis.begin(), g.axis.end(), t.begin() + 24 * gK);
+        std::copy(g.inv.begin(), g.inv.end(), t.begin() + 27 * gK);
+        std::copy(g.layers.begin(), g.layers.end(), t.begin() + 30 * gK);
+        for (uint32_t ch = 0; ch < 3; ++ch)
+            if (guide_fits(g.axis.data() + ch, g.K, 3)) {
+                uint32_t guide[kGuide];
+                fill_guide(g.axis.data() + ch, g.K, 3, guide);
+                std::memcpy(t.data() + 39 * gK + ch * kGuide, guide, sizeof guide);
+            }
+        upload(pool, s, p.dev.grain, t.data(), t.size() * sizeof(float));
     }
     const PrintSetup& pr = *p.print;
     if (!pr.paper_tab.empty()) upload(pool, s, p.dev.paper, pr.paper_tab.data(), pr.paper_tab.size() * sizeof(float));
@@ -491,6 +552,8 @@ DevelopPlan develop_plan(const RenderCtx& ctx, const Pipeline& p, uint32_t w, ui
     da.cy = da.cx + 2 * size_t(f.K);
     da.K = f.K;
     da.cgrid = axis_grid(f.cx.data(), f.K, 1);
+    da.curve4 = da.cx + 8 * size_t(f.K);
+    da.curve_last = f.cx[f.K - 1];
     da.width = w;
     da.counts_out = counts_out;
     da.lam_out = lam_out;
@@ -517,15 +580,32 @@ DevelopPlan develop_plan(const RenderCtx& ctx, const Pipeline& p, uint32_t w, ui
             da.sat_d[l * 3 + c] = f32(kc.sat_d[l][c]);
             da.count[l * 3 + c] = f32(kc.count[l][c]);
             da.unit[l * 3 + c] = da.sat_d[l * 3 + c] / da.count[l * 3 + c];
+            da.rcp_sat_d[l * 3 + c] = 1.0f / da.sat_d[l * 3 + c];
+            const uint64_t p0 = uint64_t(SPK_PHILOX_M0) * (uint32_t(SPK_STREAM_GRAIN(c, l)) ^ film_seed);
+            da.stream_hi[c * 3 + l] = uint32_t(p0 >> 32);
+            da.stream_lo[c * 3 + l] = uint32_t(p0);
         }
     if (g->sublayers) {
         da.mode = 0;  // SUM
         da.shift = 1;
         da.gK = g->K;
-        da.axis = p.dev.gaxis.as<float>();
-        da.ginv = p.dev.ginv.as<float>();
-        da.layers = p.dev.glayers.as<float>();
-        for (uint32_t c = 0; c < 3; ++c) da.ggrid[c] = axis_grid(g->axis.data() + c, g->K, 3);
+        da.layer8 = p.dev.grain.as<float>();
+        da.axis = da.layer8 + 24 * size_t(g->K);
+        da.ginv = da.layer8 + 27 * size_t(g->K);
+        da.layers = da.layer8 + 30 * size_t(g->K);
+        da.guide = reinterpret_cast<const uint32_t*>(da.layer8 + 39 * size_t(g->K));
+        // the packed kernel's quotients by spk_div_normal: far from overflow and underflow
+        da.packed = da.cgrid.active;
+        for (int i = 0; i < 9; ++i)
+            da.packed = da.packed && da.sat_d[i] > 0x1p-40f && da.sat_d[i] < 0x1p40f && da.count[i] > 0x1p-40f &&
+                        da.count[i] < 0x1p40f;
+        for (uint32_t c = 0; c < 3; ++c) {
+            da.ggrid[c] = axis_grid(g->axis.data() + c, g->K, 3);
+            da.axis_last[c] = g->axis[3 * (size_t(g->K) - 1) + c];
+            da.guide_x0[c] = g->axis[c];
+            da.guide_s[c] = guide_scale(da.guide_x0[c], da.axis_last[c]);
+            da.packed = da.packed && guide_fits(g->axis.data() + c, g->K, 3);
+        }
     } else {
         da.mode = 2;  // SIMPLE
     }
@@ -595,6 +675,7 @@ Plane dir_couplers(RenderCtx& ctx, const Pipeline& p, const Plane& H, DevelopArg
         if (core) lincomb(ctx, Vec3{1.0, 1.0, 1.0}, core, Vec3{1.0, 1.0, 1.0}, &chi, chi);
     }
     da.cy = da.cx + 5 * size_t(f.K);
+    da.curve4 += 3 * 4 * size_t(f.K);
     da.chi = chi.data();
     return chi;
 }

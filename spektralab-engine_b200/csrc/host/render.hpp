@@ -20,8 +20,10 @@ namespace spkb {
 struct DeviceTables {
     DevBuffer table;              // L x L spectral table, float4 texels (R, G, B, 0)
     DevBuffer patches;            // the same as (L - 1)^2 patches of 4 x 4 RGB texels (kPatchFloats each)
-    DevBuffer curves;             // x[K] | inv[K] | y[3K] | y0[3K] (the DIR couplers' pre-inverted curve)
-    DevBuffer gaxis, ginv, glayers;
+    DevBuffer curves;             // x[K] | inv[K] | y[3K] | y0[3K] (the DIR couplers' pre-inverted curve), then
+                                  // y and y0 again as [c][k] entries of 4 floats (DevelopArgs::curve4)
+    DevBuffer grain;              // entries [c][k] of 8 floats (DevelopArgs::layer8) | axis[3K] | inv[3K] | layers[9K] |
+                                  // the interval guide (kGuide words per channel, DevelopArgs::guide)
     DevBuffer paper;              // x[K] | r[K] | y[K][3]
     DevBuffer cmax;               // 64 x 720
     DevBuffer edr;                // the EDR tone map's target_log2_y (binary32), when EDR is on

@@ -48,6 +48,8 @@ struct AxisGrid {
     int32_t active;
 };
 
+#define kGuide 2048u  // buckets of the grain layers' interval guide, per channel
+
 // Film-side point work after halation: log10 exposure, density curves, grain draw.
 struct DevelopArgs {
     // curves: x[K], inv[K], y[3K] (channel-major)
@@ -68,11 +70,26 @@ struct DevelopArgs {
     float inv_n_sub;
     float dmin_l[9], sat_d[9], count[9];
     float unit[9];        // sat_d / count, the binary32 quotient (a draw's density per grain before saturation)
+    float rcp_sat_d[9];   // 1 / sat_d, the binary32 reciprocal
+    // Philox: the second round's product M0 (stream ^ seed) of each draw's stream, [c * 3 + l]
+    uint32_t stream_hi[9], stream_lo[9];
     float uniformity[3];
     float dmin_c[3];
     const float* axis;    // [k*3 + c]
     const float* ginv;    // [k*3 + c]
     const float* layers;  // [(k*3 + l)*3 + c]
+    // The same tables as one entry per interval, read with one load, for axes that rise (packed):
+    // curve4[c * K + k] = {x, inv, y, y(k+1) - y}; layer8[c * gK + k] = {axis, ginv, then value and step to the
+    // next point of the three sub-layers}. The last entry holds the end values with zero inv. The curves'
+    // axis has its direct index (cgrid); the densities' intervals come from kGuide buckets of equal width
+    // per channel: guide[c * kGuide + b] = first | last << 16, the intervals that a value of bucket
+    // b = min(int((v - guide_x0) guide_s), kGuide - 1) can lie in.
+    const float* curve4;
+    const float* layer8;
+    const uint32_t* guide;
+    int32_t packed;
+    float curve_last, axis_last[3];  // the axes' last points
+    float guide_x0[3], guide_s[3];
     uint32_t width;       // pixel index = y * width + x keys the draws
     float* counts_out;    // test hook: the Poisson counts, [pixel][c][l]; nullptr in renders
     float* lam_out;       // test hook: the draws' lambdas, [pixel][c][l] (sub-layer grain); nullptr in renders
