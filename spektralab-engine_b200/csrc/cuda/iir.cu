@@ -19,11 +19,15 @@
 //             loaded afresh for every mixture component, blurred and written to the component's plane.
 // k_iir_cols: one CTA per strip of 4 pixel columns (12 lines); every component's row result blurred
 //             down the columns in turn; the mixture accumulated as the reference's fused passes do
-//             (acc = 0 + w0 y0, acc = acc + w_k y_k) and the halation mix raw := a raw + b acc written
-//             in place of raw; a plain blur (one component) stores its lines as they are.
-//             A full strip (frame width a multiple of 4) comes into shared memory by TMA: the component's
-//             plane is a 2-D tensor (3 w floats x h rows), and the strip is a column of 12-float boxes of up
-//             to 256 rows, all completing on one mbarrier. Its waits are bounded: one that gives up counts
+//             (acc = 0 + w0 y0, acc = acc + w_k y_k) in tensor memory, and the halation mix raw := a raw +
+//             b acc written in place of raw; a plain blur (one component) stores its lines as they are.
+//             A strip comes into shared memory by TMA: the component's plane, its rows padded to a multiple
+//             of 4 pixels, is a 2-D tensor (3 pitch floats x h rows), and the strip is a column of 12-float
+//             boxes of up to 256 rows, all completing on one mbarrier.
+//             Column pass, the sum in a global plane and scalar copies at odd widths before: 3840 x 2160, two
+//             components 0.289 -> 0.259 ms; 6000 x 4000, three 1.70 -> 1.31; 1999 x 1333, three 0.339 -> 0.143.
+//             At 6000 x 4000 the loads take 0.29 ms of it, raw 0.28, the recurrences the rest (one strip of
+//             twelve warps per SM; the 32-to-64-bit conversions' unit is the busiest in that phase). Its waits are bounded: one that gives up counts
 //             itself (g_iir_gave_up), waits again under the full limit for the copies in flight, and if
 //             even they never land the CTA loads this and every later strip with plain copies.
 #include <cuda.h>
@@ -54,6 +58,7 @@ constexpr int kColLines = 3 * kColPixels;
 constexpr int kSegCols = SPKB_IIR_SEG_COLS;  // segments per column line (32: two 4K strips per SM)
 static_assert(kSegCols <= (1 << kIirScanSteps), "the carry scan composes at most 2^kIirScanSteps segments");
 constexpr int kColThreads = kColLines * kSegCols;
+constexpr int kColBlocks = 2;  // resident strips the register allocation allows (a 4K column pass holds two)
 
 // The column pass's tensor maps, one per component plane, and the strip's box geometry: `boxes` boxes of
 // `box_rows` rows (a multiple of 8, at most 256) cover the frame's rows; the strip buffer holds
@@ -62,7 +67,8 @@ struct IirColMaps {
     CUtensorMap map[SPKB_MAX_COMPONENTS];
     long long wait_limit;  // SM clocks a strip wait may take before it gives up
     uint32_t box_rows, boxes;
-    uint32_t use_tma;      // 0: plain copies (a width that is not a multiple of 4, or no tensor map)
+    uint32_t use_tma;      // 0: plain copies (a pitch that is not a multiple of 4, or no tensor map)
+    uint32_t tmem_cols;    // tensor-memory columns of the mixture's sum; 0: one component, no sum to keep
 };
 
 #ifndef SPKB_IIR_COL_TMA
@@ -143,35 +149,42 @@ struct Coef {
     double B, B1, B2, B3;
 };
 
-__device__ __forceinline__ double step(const Coef& k, double x, double s1, double s2, double s3) {
-    // the oldest state first and the newest last: each state is j steps old when it enters the j-th
-    // multiply-add from the end, so the chain costs one multiply-add latency per sample
-    return fma(k.B1, s1, fma(k.B2, s2, fma(k.B3, s3, k.B * x)));
-}
+// A step of the recurrence takes the oldest state first and the newest last: each state is j steps old when
+// it enters the j-th multiply-add from the end, so the chain costs one multiply-add latency per sample.
+// One pass over the segment [a, b) of a line in shared memory (element i at base[i * stride]), ascending or
+// descending. Zero-state run: returns the end state. Writing run: from the state given, stores float(w)
+// back. Samples go in chunks of kRunChunk, loaded, converted and scaled ahead of the chain, so that a step
+// waits for the one multiply-add that takes the newest state.
+constexpr int kRunChunk = 8;
 
-// Forward pass over one segment [a, b) of a line in shared memory (element i at base[i * stride]).
-// Zero-state run: returns the end state. Writing run: from `in` state, stores float(w) back.
-__device__ __forceinline__ void seg_forward(const Coef& k, float* base, int stride, int a, int b, double& s1,
-                                            double& s2, double& s3, bool write) {
-#pragma unroll 4
-    for (int i = a; i < b; ++i) {
-        const double t = step(k, double(base[i * stride]), s1, s2, s3);
+template <bool FORWARD, bool WRITE>
+__device__ __forceinline__ void seg_run(const Coef& k, float* base, int stride, int a, int b, double& s1, double& s2,
+                                        double& s3) {
+    const int n = b - a, dir = FORWARD ? stride : -stride;
+    float* p = base + (FORWARD ? a : b - 1) * stride;
+    const auto chain = [&](double kx) {
+        const double t = fma(k.B1, s1, fma(k.B2, s2, fma(k.B3, s3, kx)));
         s3 = s2;
         s2 = s1;
         s1 = t;
-        if (write) base[i * stride] = float(t);
+        return float(t);
+    };
+    int i = 0;
+#pragma unroll 1
+    for (; i + kRunChunk <= n; i += kRunChunk, p += kRunChunk * dir) {
+        double kx[kRunChunk];
+#pragma unroll
+        for (int j = 0; j < kRunChunk; ++j) kx[j] = k.B * double(p[j * dir]);
+#pragma unroll
+        for (int j = 0; j < kRunChunk; ++j) {
+            const float v = chain(kx[j]);
+            if (WRITE) p[j * dir] = v;
+        }
     }
-}
-
-__device__ __forceinline__ void seg_backward(const Coef& k, float* base, int stride, int a, int b, double& s1,
-                                             double& s2, double& s3, bool write) {
-#pragma unroll 4
-    for (int i = b - 1; i >= a; --i) {
-        const double t = step(k, double(base[i * stride]), s1, s2, s3);
-        s3 = s2;
-        s2 = s1;
-        s1 = t;
-        if (write) base[i * stride] = float(t);
+#pragma unroll 1
+    for (; i < n; ++i, p += dir) {
+        const float v = chain(k.B * double(*p));
+        if (WRITE) *p = v;
     }
 }
 
@@ -222,7 +235,7 @@ __device__ __forceinline__ void edge_fold(const Coef& k, float* base, int e, int
 // handles line t / nseg, segment t % nseg when seg_major, else line t % nlines, segment t / nlines; the
 // channel of line j is 3 comp + j % 3. carry: shared scratch of 3 * nlines * nseg doubles, component i of
 // thread t's segment at carry[i * nlines * nseg + t].
-__device__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, const IirLaunch& q, int comp,
+__device__ __forceinline__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, const IirLaunch& q, int comp,
                            double* carry, bool seg_major) {
     const int t = threadIdx.x;
     const int line = seg_major ? t / nseg : t % nlines;
@@ -243,7 +256,7 @@ __device__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, c
     if (active && a < n) {
         double s1 = 0.0, s2 = 0.0, s3 = 0.0;
         if (seg == 0 && !adj) s1 = s2 = s3 = double(base[0]);
-        seg_forward(k, base, pitch, a, b, s1, s2, s3, false);
+        seg_run<true, false>(k, base, pitch, a, b, s1, s2, s3);
         cs[0] = s1;
         cs[nt] = s2;
         cs[2 * nt] = s3;
@@ -262,7 +275,7 @@ __device__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, c
             s2 = prev[nt];
             s3 = prev[2 * nt];
         }
-        seg_forward(k, base, pitch, a, b, s1, s2, s3, true);
+        seg_run<true, true>(k, base, pitch, a, b, s1, s2, s3);
     }
     __syncthreads();
     if (adj) {
@@ -275,7 +288,7 @@ __device__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, c
     if (active && a < n) {
         double s1 = 0.0, s2 = 0.0, s3 = 0.0;
         if (seg == last && !adj) s1 = s2 = s3 = double(base[(n - 1) * pitch]);
-        seg_backward(k, base, pitch, a, b, s1, s2, s3, false);
+        seg_run<false, false>(k, base, pitch, a, b, s1, s2, s3);
         cs[0] = s1;
         cs[nt] = s2;
         cs[2 * nt] = s3;
@@ -292,7 +305,7 @@ __device__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, c
             s2 = prev[nt];
             s3 = prev[2 * nt];
         }
-        seg_backward(k, base, pitch, a, b, s1, s2, s3, true);
+        seg_run<false, true>(k, base, pitch, a, b, s1, s2, s3);
     }
     __syncthreads();
     if (adj) {
@@ -310,39 +323,183 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__global__ void __launch_bounds__(kRowThreads) k_iir_rows(const float* __restrict__ in, IirPlanes outs, uint32_t w,
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+__global__ void __launch_bounds__(kRowThreads) k_iir_rows(const float* __restrict__ in, const __grid_constant__ IirPlanes outs, uint32_t w,
                                                           uint32_t h, const __grid_constant__ IirMixture mix) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t y = blockIdx.x;
     if (y >= h) return;
-    const int n3 = int(3 * w);
-    const int n3r = (n3 + 3) & ~3;  // keeps carry 16-byte aligned
+    const int n3 = int(3 * w), p3 = int(3 * mix.pitch);
+    const int n3r = (p3 + 3) & ~3;  // keeps carry 16-byte aligned
     float* work = reinterpret_cast<float*>(smem);
     double* carry = reinterpret_cast<double*>(work + n3r);
     const float* src = in + size_t(y) * n3;
-    const bool vec = (n3 & 3) == 0;  // rows start on 16-byte boundaries
+    const bool vec = (n3 & 3) == 0;  // the source's rows start on 16-byte boundaries
+    for (int i = n3 + int(threadIdx.x); i < p3; i += blockDim.x) work[i] = 0.0f;  // the padding
     for (int c = 0; c < int(mix.ncomp); ++c) {
         // each component blurs the row afresh: the source row is read again (from L2 after the first)
         if (vec) {
             for (int i = threadIdx.x; i < n3 / 4; i += blockDim.x) cp_async16(work + 4 * i, src + 4 * i);
-            cp_async_wait_all();
         } else {
-            for (int i = threadIdx.x; i < n3; i += blockDim.x) work[i] = src[i];
+#pragma unroll 4
+            for (int i = threadIdx.x; i < n3; i += blockDim.x) cp_async4(work + i, src + i);
         }
+        cp_async_wait_all();
         __syncthreads();
         blur_lines(work, 3, 3, int(w), kSegRows, mix.rows, c, carry, true);
-        float* dst = outs.p[c] + size_t(y) * n3;
-        if (vec) {
-            for (int i = threadIdx.x; i < n3 / 4; i += blockDim.x)
+        float* dst = outs.p[c] + size_t(y) * p3;
+        if ((p3 & 3) == 0) {
+            for (int i = threadIdx.x; i < p3 / 4; i += blockDim.x)
                 reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(work)[i];
         } else {
-            for (int i = threadIdx.x; i < n3; i += blockDim.x) dst[i] = work[i];
+            for (int i = threadIdx.x; i < p3; i += blockDim.x) dst[i] = work[i];
         }
         __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(kColThreads) k_iir_cols(float* raw, IirPlanes hs, float* acc, uint32_t w, uint32_t h,
+// The mixture's sum lives in tensor memory, used as the strip's scratch: the 12 n floats that a global plane
+// would have to hold (written, read and written again for every component but one) do not fit beside
+// the strip in shared memory, but they fill at most 435 of the SM's 512 columns of 128 words. Quad i (four
+// floats of a strip row, three to a row) belongs to thread i % kColThreads, which keeps it in its own lane at
+// columns 4 (i / 128) ..: warp w's lanes start at 32 (w % 4), and its 32 quads of turn k are 384 k + 32 w ...
+// Only the owner ever reads a quad, so no barrier orders the accesses.
+__device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ float4 tmem_ld4(uint32_t taddr) {
+    uint32_t r[4];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+        : "r"(taddr)
+        : "memory");
+    return make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const float4& v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr),
+                 "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w))
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+constexpr int kQuads = kColLines / 4, kQuadRows = kColThreads / kQuads;
+static_assert(kQuads == 3 && kColThreads == 384, "the tensor-memory layout above");
+
+// One thread's weights of its four channels
+struct QuadWeights {
+    float w[4];
+};
+__device__ __forceinline__ QuadWeights quad_weights(const float (&w)[3]) {
+    const int j = 4 * (int(threadIdx.x) % kQuads);
+    return {{w[j % 3], w[(j + 1) % 3], w[(j + 2) % 3], w[j % 3]}};
+}
+__device__ __forceinline__ float4 sum_quad(const QuadWeights& wc, const float4& v, bool first, uint32_t taddr) {
+    if (first) return make_float4(0.0f + wc.w[0] * v.x, 0.0f + wc.w[1] * v.y, 0.0f + wc.w[2] * v.z, 0.0f + wc.w[3] * v.w);
+    const float4 a = tmem_ld4(taddr);
+    return make_float4(a.x + wc.w[0] * v.x, a.y + wc.w[1] * v.y, a.z + wc.w[2] * v.z, a.w + wc.w[3] * v.w);
+}
+
+// mix_a raw + mix_b sum with the product of x unrounded. Frames whose width is a multiple of 4 take x = mix_a
+// raw and the others x = mix_b sum: either is within the sum's rounding, and each keeps the bits that the
+// renders of its frames have always had.
+__device__ __forceinline__ float mix2(float mx, float x, float my, float y) { return __fmaf_rn(mx, x, __fmul_rn(my, y)); }
+
+// The blurred strip of component c joins the sum: acc := 0 + w v or acc + w v. The result goes back to the
+// tensor memory, or (to_strip) over the strip. Every lane of a warp with a quad left takes part in the
+// tensor-memory accesses; the quads past the frame's rows are the strip buffer's padding or its last row.
+__device__ __forceinline__ void strip_sum(float* strip, int n, const IirMixture& mix, int c, uint32_t tmem, bool to_strip) {
+    const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads, last = n - 1;
+    const QuadWeights wc = quad_weights(mix.weight[c]);
+    uint32_t taddr = tmem + (uint32_t(32 * (warp & 3)) << 16) + 4u * uint32_t(warp >> 2);
+    for (int q0 = 32 * warp, row = int(threadIdx.x) / kQuads; q0 < kQuads * n; q0 += kColThreads, row += kQuadRows, taddr += 12u) {
+        float4* at = reinterpret_cast<float4*>(strip + size_t(min(row, last)) * kColLines + 4 * qd);
+        const float4 a = sum_quad(wc, *at, c == 0, taddr);
+        if (!to_strip) tmem_st4(taddr, a);
+        else if (row <= last) *at = a;
+    }
+    if (!to_strip) tmem_wait_st();
+}
+
+// raw := mix_a raw + mix_b (the sum after the last component c), or the strip as it is (plain), in float4.
+// A thread steps down the rows kStoreBatch at a time, their reads issued before the first store.
+constexpr int kStoreBatch = 4;
+
+__device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, size_t pitch, int n, const IirMixture& mix,
+                                             int c, uint32_t tmem) {
+    const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads;
+    const QuadWeights wc = quad_weights(mix.weight[c]), ma = quad_weights(mix.mix_a), mb = quad_weights(mix.mix_b);
+    const bool plain = mix.plain != 0;
+    uint32_t taddr = tmem + (uint32_t(32 * (warp & 3)) << 16) + 4u * uint32_t(warp >> 2);
+    int row = int(threadIdx.x) / kQuads;
+    float* out = raw + size_t(row) * pitch + 4 * qd;
+    const size_t step = size_t(kQuadRows) * pitch;
+    for (int q0 = 32 * warp; q0 < kQuads * n; q0 += kStoreBatch * kColThreads) {
+        float4 rw[kStoreBatch];
+        if (!plain) {
+#pragma unroll
+            for (int u = 0; u < kStoreBatch; ++u)
+                if (row + u * kQuadRows < n) rw[u] = *reinterpret_cast<const float4*>(out + u * step);
+        }
+#pragma unroll
+        for (int u = 0; u < kStoreBatch; ++u) {
+            if (q0 + u * kColThreads >= kQuads * n) break;
+            const int r = min(row, n - 1);
+            float4 v = *reinterpret_cast<const float4*>(strip + size_t(r) * kColLines + 4 * qd);
+            if (!plain) {
+                const float4 a = sum_quad(wc, v, c == 0, taddr);
+                v.x = mix2(ma.w[0], rw[u].x, mb.w[0], a.x);
+                v.y = mix2(ma.w[1], rw[u].y, mb.w[1], a.y);
+                v.z = mix2(ma.w[2], rw[u].z, mb.w[2], a.z);
+                v.w = mix2(ma.w[3], rw[u].w, mb.w[3], a.w);
+            }
+            if (row < n) *reinterpret_cast<float4*>(out) = v;
+            row += kQuadRows;
+            out += step;
+            taddr += 12u;
+        }
+    }
+}
+
+// The same from a strip that holds the sum (or the plain blur) to a raw whose rows are not aligned, or a
+// strip cut by the frame's edge: a float at a time, nl to a row
+__device__ __forceinline__ void strip_to_raw_scalar(const float* strip, float* raw, size_t pitch, int nl, int n,
+                                                    const IirMixture& mix) {
+    constexpr int kStep = kColThreads / kColLines, kBatch = 8;
+    const int j = int(threadIdx.x) % kColLines;
+    if (j >= nl) return;
+    const float ma = mix.mix_a[j % 3], mb = mix.mix_b[j % 3];
+    for (int r = int(threadIdx.x) / kColLines; r < n; r += kBatch * kStep) {
+        float rw[kBatch];
+        if (!mix.plain) {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+                if (r + u * kStep < n) rw[u] = raw[size_t(r + u * kStep) * pitch + j];
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int row = r + u * kStep;
+            if (row >= n) break;
+            const float a = strip[size_t(row) * kColLines + j];
+            raw[size_t(row) * pitch + j] = mix.plain ? a : mix2(mb, a, ma, rw[u]);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kColThreads, kColBlocks) k_iir_cols(float* raw, const __grid_constant__ IirPlanes hs, uint32_t w, uint32_t h,
                                                           const __grid_constant__ IirMixture mix,
                                                           const __grid_constant__ IirColMaps maps) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -356,11 +513,10 @@ __global__ void __launch_bounds__(kColThreads) k_iir_cols(float* raw, IirPlanes 
     float* strip = reinterpret_cast<float*>(smem);
     double* carry = reinterpret_cast<double*>(strip + rows_alloc * kColLines);
     const uint32_t bar = smem_addr(carry + size_t(kColLines) * kSegCols * 3);
-    const size_t pitch = 3 * size_t(w);
+    const size_t pitch = 3 * size_t(mix.pitch), raw_pitch = 3 * size_t(w);
     const size_t off = 3 * size_t(x0);
-    // a full strip of a frame whose width is a multiple of 4: every strip row is three aligned float4
-    const bool vec = px == kColPixels && (w & 3u) == 0;
-    constexpr int kQuads = kColLines / 4;
+    // rows of the component planes and the sum (vec), of raw (raw_vec), as three aligned float4 a strip row
+    const bool vec = (mix.pitch & 3u) == 0, raw_vec = px == kColPixels && (w & 3u) == 0;
     bool tma = vec && maps.use_tma != 0;  // the same in every thread of the CTA
     if (tma) {
         if (threadIdx.x == 0) {
@@ -368,6 +524,18 @@ __global__ void __launch_bounds__(kColThreads) k_iir_cols(float* raw, IirPlanes 
             fence_mbar_init();
         }
         __syncthreads();
+    }
+    const uint32_t tmem_slot = bar + 8;
+    uint32_t tmem = 0;
+    if (maps.tmem_cols != 0) {
+        if (threadIdx.x < 32) {
+            tmem_alloc(tmem_slot, maps.tmem_cols);
+            tmem_relinquish();
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
     }
     for (int c = 0; c < int(mix.ncomp); ++c) {
         const float* src = hs.p[c];
@@ -407,72 +575,31 @@ __global__ void __launch_bounds__(kColThreads) k_iir_cols(float* raw, IirPlanes 
         }
         __syncthreads();
         blur_lines(strip, kColLines, kColLines, n, kSegCols, mix.cols, c, carry, false);
-        const bool first = c == 0, last = c + 1 == int(mix.ncomp);
-        if (mix.plain) {
-            // a plain blur (one component): the blurred lines as they are
-            if (vec) {
-                for (int i = threadIdx.x; i < n * kQuads; i += blockDim.x) {
-                    const int r = i / kQuads, qd = i - r * kQuads;
-                    *reinterpret_cast<float4*>(raw + size_t(r) * pitch + off + 4 * qd) =
-                        *reinterpret_cast<const float4*>(strip + size_t(r) * kColLines + 4 * qd);
-                }
-            } else {
-                for (int i = threadIdx.x; i < n * kColLines; i += blockDim.x) {
-                    const int r = i / kColLines, j = i % kColLines;
-                    if (j < nl) raw[size_t(r) * pitch + off + j] = strip[i];
-                }
-            }
-        } else if (vec) {
-            for (int i = threadIdx.x; i < n * kQuads; i += blockDim.x) {
-                const int r = i / kQuads, qd = i - r * kQuads;
-                const size_t o = size_t(r) * pitch + off + 4 * qd;
-                const float4 v = *reinterpret_cast<const float4*>(strip + size_t(r) * kColLines + 4 * qd);
-                const float vv[4] = {v.x, v.y, v.z, v.w};
-                float av[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                if (!first) {
-                    const float4 p = *reinterpret_cast<const float4*>(acc + o);
-                    av[0] = p.x;
-                    av[1] = p.y;
-                    av[2] = p.z;
-                    av[3] = p.w;
-                }
-                float4 rw = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (last) rw = *reinterpret_cast<const float4*>(raw + o);
-                float rr[4] = {rw.x, rw.y, rw.z, rw.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int ch3 = (4 * qd + e) % 3;
-                    const float wc = mix.weight[c][ch3];
-                    av[e] = first ? 0.0f + wc * vv[e] : av[e] + wc * vv[e];
-                    if (last) rr[e] = mix.mix_a[ch3] * rr[e] + mix.mix_b[ch3] * av[e];
-                }
-                if (last) *reinterpret_cast<float4*>(raw + o) = make_float4(rr[0], rr[1], rr[2], rr[3]);
-                else *reinterpret_cast<float4*>(acc + o) = make_float4(av[0], av[1], av[2], av[3]);
-            }
+        if (mix.plain == 0 && c + 1 < int(mix.ncomp)) {
+            strip_sum(strip, n, mix, c, tmem, false);
+        } else if (raw_vec) {
+            strip_to_raw(strip, raw + off, raw_pitch, n, mix, c, tmem);
         } else {
-            for (int i = threadIdx.x; i < n * kColLines; i += blockDim.x) {
-                const int r = i / kColLines, j = i % kColLines;
-                if (j >= nl) continue;
-                const size_t o = size_t(r) * pitch + off + j;
-                const float v = strip[i];
-                const float wc = mix.weight[c][j % 3];
-                const float a = first ? 0.0f + wc * v : acc[o] + wc * v;
-                if (last) {
-                    const float m0 = mix.mix_a[j % 3], m1 = mix.mix_b[j % 3];
-                    raw[o] = m0 * raw[o] + m1 * a;
-                } else {
-                    acc[o] = a;
-                }
+            if (mix.plain == 0) {
+                strip_sum(strip, n, mix, c, tmem, true);
+                __syncthreads();
             }
+            strip_to_raw_scalar(strip, raw + off, raw_pitch, nl, n, mix);
         }
         __syncthreads();
+    }
+    if (maps.tmem_cols != 0) {
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        if (threadIdx.x < 32) tmem_dealloc(tmem, maps.tmem_cols);
     }
 }
 
 }  // namespace
 
-size_t iir_rows_smem(uint32_t w) {
-    const size_t n3r = (3 * size_t(w) + 3) & ~size_t(3);
+size_t iir_rows_smem(uint32_t pitch) {
+    const size_t n3r = (3 * size_t(pitch) + 3) & ~size_t(3);
     return n3r * sizeof(float) + size_t(3) * kSegRows * 3 * sizeof(double);
 }
 
@@ -491,7 +618,7 @@ ColBoxes col_boxes(uint32_t h) {
 size_t iir_cols_smem(uint32_t h) {
     const ColBoxes cb = col_boxes(h);
     return size_t(cb.rows) * cb.boxes * kColLines * sizeof(float) + size_t(kColLines) * kSegCols * 3 * sizeof(double) +
-           sizeof(uint64_t);
+           2 * sizeof(uint64_t);  // the mbarrier, the tensor memory's base
 }
 
 // The column segment length: at least n / nseg, and with nlines L = nlines (mod 32), so that a warp's
@@ -515,11 +642,23 @@ int iir_row_seg_len(uint32_t w) {
 }
 int iir_col_seg_len(uint32_t h) { return seg_len(h, kSegCols, kColLines); }
 
-bool iir_mixture_fits(uint32_t w, uint32_t h) {
+namespace {
+size_t smem_limit() {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    return iir_rows_smem(w) <= size_t(optin) && iir_cols_smem(h) <= size_t(optin);
+    return size_t(optin);
+}
+}  // namespace
+
+bool iir_mixture_fits(uint32_t w, uint32_t h) {
+    const size_t limit = smem_limit();
+    return iir_rows_smem(w) <= limit && iir_cols_smem(h) <= limit;
+}
+
+uint32_t iir_pitch(uint32_t w) {
+    const uint32_t padded = (w + 3u) & ~3u;
+    return padded == w || iir_rows_smem(padded) <= smem_limit() ? padded : w;
 }
 
 namespace {
@@ -544,11 +683,11 @@ EncodeTiled encode_tiled() {
 
 std::atomic<long long> g_wait_limit{0};  // set_iir_wait_limit: 0 the full limit
 
-// The tensor maps of the column pass's component planes: each a 2-D tensor of 3 w floats x h rows (row
-// pitch 12 w bytes), read in 12 x box_rows boxes. False (plain copies) for a width that is not a multiple
-// of 4 (the rows and the strips' x coordinates would leave 16-byte alignment), a plane not on a 16-byte
+// The tensor maps of the column pass's component planes, `pitch` pixels a row: each a 2-D tensor of 3 pitch
+// floats x h rows, read in 12 x box_rows boxes. False (plain copies) for a pitch that is not a multiple of 4
+// (the rows and the strips' x coordinates would leave 16-byte alignment), a plane not on a 16-byte
 // boundary, or a map the driver refuses.
-bool col_maps(IirColMaps& maps, const IirPlanes& planes, uint32_t ncomp, uint32_t w, uint32_t h) {
+bool col_maps(IirColMaps& maps, const IirPlanes& planes, uint32_t ncomp, uint32_t pitch, uint32_t h) {
     const ColBoxes cb = col_boxes(h);
     maps.box_rows = cb.rows;
     maps.boxes = cb.boxes;
@@ -556,9 +695,9 @@ bool col_maps(IirColMaps& maps, const IirPlanes& planes, uint32_t ncomp, uint32_
     maps.wait_limit = lim > 0 ? lim : kWaitCycles;
     maps.use_tma = 0;
     const EncodeTiled enc = encode_tiled();
-    if (!kColTma || !enc || (w & 3u) != 0u) return false;
-    const cuuint64_t dims[2] = {cuuint64_t(3) * w, h};
-    const cuuint64_t strides[1] = {cuuint64_t(3) * w * sizeof(float)};
+    if (!kColTma || !enc || (pitch & 3u) != 0u) return false;
+    const cuuint64_t dims[2] = {cuuint64_t(3) * pitch, h};
+    const cuuint64_t strides[1] = {cuuint64_t(3) * pitch * sizeof(float)};
     const cuuint32_t box[2] = {cuuint32_t(kColLines), cb.rows};
     const cuuint32_t estr[2] = {1, 1};
     for (uint32_t c = 0; c < ncomp; ++c) {
@@ -583,22 +722,28 @@ uint32_t take_iir_waits_given_up(cudaStream_t s) {
     return v;
 }
 
-void iir_mixture(const float* src, float* raw, float* const* tmp, float* acc, uint32_t w, uint32_t h,
-                 const IirMixture& m, cudaStream_t s) {
+void iir_mixture(const float* src, float* raw, float* const* tmp, uint32_t w, uint32_t h, const IirMixture& m,
+                 cudaStream_t s) {
     IirPlanes planes{};
     for (uint32_t c = 0; c < m.ncomp; ++c) planes.p[c] = tmp[c];
-    const size_t sr = iir_rows_smem(w), sc = iir_cols_smem(h);
+    const size_t sr = iir_rows_smem(m.pitch), sc = iir_cols_smem(h);
     ensure_smem(reinterpret_cast<const void*>(k_iir_rows), int(sr));
     ensure_smem(reinterpret_cast<const void*>(k_iir_cols), int(sc));
     IirColMaps maps{};
-    col_maps(maps, planes, m.ncomp, w, h);
+    col_maps(maps, planes, m.ncomp, m.pitch, h);
+    if (m.ncomp > 1) {
+        // four columns for every 128 quads; allocations are powers of two from 32
+        const uint32_t need = 4u * ((3u * h + 127u) / 128u);
+        maps.tmem_cols = 32;
+        while (maps.tmem_cols < need) maps.tmem_cols *= 2;
+    }
     {
         Probe p("iir_rows", s);
         k_iir_rows<<<h, kRowThreads, sr, s>>>(src, planes, w, h, m);
     }
     {
         Probe p("iir_cols", s);
-        k_iir_cols<<<(w + kColPixels - 1) / kColPixels, kColThreads, sc, s>>>(raw, planes, acc, w, h, m, maps);
+        k_iir_cols<<<(w + kColPixels - 1) / kColPixels, kColThreads, sc, s>>>(raw, planes, w, h, m, maps);
     }
 }
 

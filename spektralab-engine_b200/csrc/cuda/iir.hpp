@@ -35,6 +35,7 @@ struct IirMixture {
     // pass stores the blurred lines as they are and never reads raw
     uint32_t plain;
     float weight[SPKB_MAX_COMPONENTS][3];
+    uint32_t pitch;  // pixels per row of the tmp planes, at least the frame's width (iir_pitch)
     float mix_a[3], mix_b[3];  // raw := mix_a raw + mix_b sum_k weight_k G_k(raw)
     IirLaunch rows, cols;
 };
@@ -43,18 +44,21 @@ struct IirPlanes {
     float* p[SPKB_MAX_COMPONENTS];
 };
 
-size_t iir_rows_smem(uint32_t w);
+size_t iir_rows_smem(uint32_t pitch);
 size_t iir_cols_smem(uint32_t h);
 int iir_row_seg_len(uint32_t w);  // segment length of the row and column passes for this frame
 int iir_col_seg_len(uint32_t h);
 bool iir_mixture_fits(uint32_t w, uint32_t h);  // both kernels' lines fit in shared memory
 
+// The row pitch of tmp, in pixels, that lets every strip of the column pass be loaded by TMA: the width rounded up to a multiple of 4 (the width itself for the
+// one or two widths whose padded row alone exceeds shared memory)
+uint32_t iir_pitch(uint32_t w);
+
 // raw := mix_a raw + mix_b sum_k weight_k G_k(src), every component recursive on every active channel
 // (an inactive channel's lines pass through G_k unchanged); src is raw itself or, for a plain blur, any
-// plane (raw := G_0(src)). tmp: ncomp planes for the row results; acc: one plane for the running sum
-// (unused for one component).
-void iir_mixture(const float* src, float* raw, float* const* tmp, float* acc, uint32_t w, uint32_t h,
-                 const IirMixture& m, cudaStream_t s);
+// plane (raw := G_0(src)). tmp: ncomp planes of m.pitch x h pixels for the row results.
+void iir_mixture(const float* src, float* raw, float* const* tmp, uint32_t w, uint32_t h, const IirMixture& m,
+                 cudaStream_t s);
 
 // Test hooks of the column pass's bounded TMA waits: the SM clocks a strip wait may take before it gives
 // up (0: the full limit, about 2 s; process-wide), and the number of waits that gave up since the last

@@ -27,6 +27,7 @@
 
 #include "../host/blur_plan.h"
 #include "../host/status.hpp"
+#include "iir.hpp"
 #include "launch.hpp"
 #include "spektralab_b200.h"
 
@@ -119,7 +120,8 @@ extern "C" SPK_API spk_status spkx_gaussian_noalloc(const float* in, float* out,
         }
         // the block-parallel kernels where the lines fit in shared memory (the other channels pass
         // through), else one thread per line
-        if (!blur_iir_block(src, out, s0, w, h, sigma3, iir, st)) {
+        const uint32_t padded = dev::iir_pitch(w), pitch = size_t(padded) * h * 3 <= dev::kMaxFloats ? padded : w;
+        if (!blur_iir_block(src, out, s0, pitch, w, h, sigma3, iir, st)) {
             const IirCoefs coefs = blur_iir_coefs(sigma3, iir);
             dev::iir_h(src, s0, w, h, coefs, st);
             dev::iir_v(s0, out, out, w, h, coefs, ACC_NONE, one, st);

@@ -366,8 +366,8 @@ void gaussian(RenderCtx& ctx, const Plane& in, const Plane& dst, const Vec3& sig
         blur_branch(sigma[2]) == Branch::Iir && dev::iir_mixture_fits(in.w, in.h)) {
         const double s3[3] = {sigma[0], sigma[1], sigma[2]};
         const bool all[3] = {true, true, true};
-        Plane tmp = make_plane(ctx.pool, in.w, in.h);
-        if (blur_iir_block(in.data(), dst.data(), tmp.data(), in.w, in.h, s3, all, ctx.stream)) return;
+        Plane tmp = make_plane(ctx.pool, dev::iir_pitch(in.w), in.h);
+        if (blur_iir_block(in.data(), dst.data(), tmp.data(), tmp.w, in.w, in.h, s3, all, ctx.stream)) return;
     }
     encode_blur(ctx, in, dst, sigma, Fuse{});
 }
@@ -454,32 +454,33 @@ bool iir_mixture_mix(RenderCtx& ctx, const Plane& raw, const std::vector<Mixture
     fill_launch(q.rows, comps, Lr);
     fill_launch(q.cols, comps, Lc);
     q.rows.adjoint = q.cols.adjoint = adjoint ? 1 : 0;
+    q.pitch = dev::iir_pitch(raw.w);
     std::vector<Plane> tmp;
     float* tp[SPKB_MAX_COMPONENTS] = {};
     for (size_t c = 0; c < comps.size(); ++c) {
-        tmp.push_back(make_plane(ctx.pool, raw.w, raw.h));
+        tmp.push_back(make_plane(ctx.pool, q.pitch, raw.h));
         tp[c] = tmp.back().data();
     }
-    Plane acc = comps.size() > 1 ? make_plane(ctx.pool, raw.w, raw.h) : Plane{};
-    dev::iir_mixture(raw.data(), raw.data(), tp, acc ? acc.data() : nullptr, raw.w, raw.h, q, ctx.stream);
+    dev::iir_mixture(raw.data(), raw.data(), tp, raw.w, raw.h, q, ctx.stream);
     return true;
 }
 
 }  // namespace
 
-bool blur_iir_block(const float* src, float* dst, float* tmp, uint32_t w, uint32_t h, const double sigma[3],
-                    const bool iir[3], cudaStream_t s) {
+bool blur_iir_block(const float* src, float* dst, float* tmp, uint32_t tmp_pitch, uint32_t w, uint32_t h,
+                    const double sigma[3], const bool iir[3], cudaStream_t s) {
     // the kernels move whole rows and strips in 16-byte pieces from the planes' bases
     auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (!aligned(src) || !aligned(dst) || !aligned(tmp) || !dev::iir_mixture_fits(w, h)) return false;
     dev::IirMixture q{};
     q.ncomp = 1;
     q.plain = 1;
+    q.pitch = tmp_pitch;
     const std::vector<MixtureComponent> one{MixtureComponent{Vec3{1.0, 1.0, 1.0}, Vec3{sigma[0], sigma[1], sigma[2]}}};
     fill_launch(q.rows, one, dev::iir_row_seg_len(w), iir);
     fill_launch(q.cols, one, dev::iir_col_seg_len(h), iir);
     float* tp[SPKB_MAX_COMPONENTS] = {tmp};
-    dev::iir_mixture(src, dst, tp, nullptr, w, h, q, s);
+    dev::iir_mixture(src, dst, tp, w, h, q, s);
     return true;
 }
 

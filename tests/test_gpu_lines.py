@@ -42,3 +42,19 @@ def test_long_lines_mixture_against_fp64(engine, lib, resources, w, h):
     f64 = setup_f64(lib, resources, delta, 200000.0 / max(w, h))["f64"]
     _, want = oracle.Oracle(f64, seed=1, halation=hal).render(img)
     np.testing.assert_allclose(neg, want, rtol=0, atol=5e-5)  # the float64 gate of the other negatives
+
+
+@pytest.mark.parametrize("w,h", [(4, 1), (5, 42), (6, 43), (7, 128), (8, 129), (12, 171), (33, 700), (130, 257), (64, 2560)])
+def test_block_mixture_against_fp64(engine, lib, resources, w, h):
+    """The block-parallel mixture of three recursive components: strips cut by the frame's edge, frames whose
+    rows are not aligned, and the edges of the sum's turns of 128 quads in tensor memory."""
+    hal = ([((1.0, 0.5, 0.25), (3.5, 4.0, 5.0)), ((0.5, 1.0, 0.75), (8, 8, 8)), ((0.25, 0.5, 1.0), (40, 30, 20))],
+           (0.3, 0.2, 0.1))
+    delta = dict(BASE, grain_active=False)
+    img = sc.synthetic_image(w, h, 9)
+    with engine.open(img, delta) as s:
+        s.set_halation(*hal)
+        neg, _ = s.develop_debug("full", 1, w, h, counts=False)
+    f64 = setup_f64(lib, resources, delta, 35000.0 / max(w, h))["f64"]
+    _, want = oracle.Oracle(f64, seed=1, halation=hal).render(img)
+    np.testing.assert_allclose(neg, want, rtol=0, atol=5e-5)  # the float64 gate of the other negatives
