@@ -129,6 +129,12 @@ constexpr uint32_t scan_tile_rows() { return 32; }
 bool fir_tile_fits(uint32_t w, uint32_t h, int r);
 void fir_tile(const float* in, float* out, uint32_t w, uint32_t h, int r, const float* taps, cudaStream_t s);
 
+// A run of a.n separable FIRs of one plane with per-channel taps, every pass of all of them in one tiled
+// kernel: out := G(in) (one component, ACC_NONE), or out := (0 or acc) + sum_k weight_k G_k(in), the terms
+// added in order. out must not alias in; acc may be out. fir_tile_fits tells for the radius a.rmax.
+void fir_mixture(const float* in, float* out, const float* acc, uint32_t w, uint32_t h, const FirMixArgs& a,
+                 cudaStream_t s);
+
 // The print and scanner stages of many frames, each in one persistent launch of `ctas` CTAs: print over
 // items of item_px pixels (item_frame / item_first per item, ordered by frame; frames in device memory),
 // the scanner over the frames' concatenated 32 x 32 tile lists (frames in device memory, ordered by

@@ -275,6 +275,16 @@ void encode_fir(RenderCtx& ctx, const Plane& in, const Plane& dst, const FirTaps
         dev::copy(tmp.data(), dst.data(), dst.pixels(), ctx.stream);
         return;
     }
+    if (!same(in, dst) && dev::fir_tile_fits(in.w, in.h, t.r)) {
+        FirMixArgs a{};
+        a.n = 1;
+        a.mode = fuse.mode;
+        a.rmax = t.r;
+        a.t[0] = t;
+        weights(fuse.weight, a.weight[0]);
+        dev::fir_mixture(in.data(), dst.data(), fuse.acc ? fuse.acc->data() : dst.data(), in.w, in.h, a, ctx.stream);
+        return;
+    }
     Plane tmp = make_plane(ctx.pool, in.w, in.h);
     dev::fir_v(in.data(), tmp.data(), in.w, in.h, t, ctx.stream);
     float w[3];
@@ -375,11 +385,31 @@ void gaussian(RenderCtx& ctx, const Plane& in, const Plane& dst, const Vec3& sig
 void gaussian_mixture(RenderCtx& ctx, const Plane& in, const Plane& out, const std::vector<MixtureComponent>& comps) {
     if (comps.empty()) fail_internal("empty mixture");
     Plane acc = same(in, out) ? make_plane(ctx.pool, in.w, in.h) : out;
+    const bool no_iir[3] = {false, false, false};
+    const auto all_fir = [](const MixtureComponent& m) {
+        return blur_branch(m.sigma[0]) != Branch::Iir && blur_branch(m.sigma[1]) != Branch::Iir &&
+               blur_branch(m.sigma[2]) != Branch::Iir;
+    };
     for (size_t k = 0; k < comps.size(); ++k) {
         const MixtureComponent& m = comps[k];
         const bool ident = !(m.sigma[0] > 0.0) && !(m.sigma[1] > 0.0) && !(m.sigma[2] > 0.0);
         if (k == 0 && ident) {
             lincomb(ctx, Vec3{0.0, 0.0, 0.0}, in, m.weight, &in, acc);
+            continue;
+        }
+        // a run of components with no recursive channel: one launch for all of them
+        FirMixArgs a{};
+        size_t j = k;
+        for (; j < comps.size() && a.n < SPKB_MAX_COMPONENTS && all_fir(comps[j]); ++j) {
+            a.t[a.n] = fir_taps(comps[j].sigma, no_iir);
+            a.rmax = std::max(a.rmax, a.t[a.n].r);
+            weights(comps[j].weight, a.weight[a.n]);
+            ++a.n;
+        }
+        if (a.n > 0 && dev::fir_tile_fits(in.w, in.h, a.rmax)) {
+            a.mode = k == 0 ? ACC_ZERO : ACC_PLANE;
+            dev::fir_mixture(in.data(), acc.data(), acc.data(), in.w, in.h, a, ctx.stream);
+            k = j - 1;
             continue;
         }
         Fuse f;

@@ -30,6 +30,15 @@ struct FirTaps {
     float taps[3][2 * SPKB_FIR_MAX_R + 1];
 };
 
+// A run of FIR Gaussians of one plane and how they join the mixture's sum (fir_mixture).
+struct FirMixArgs {
+    uint32_t n;
+    int32_t mode;  // AccMode of the first component; the later ones add to the sum
+    int32_t rmax;  // the largest radius
+    FirTaps t[SPKB_MAX_COMPONENTS];
+    float weight[SPKB_MAX_COMPONENTS][3];
+};
+
 // One recursive (Young-van Vliet) Gaussian: binary64 coefficients per channel; mask bit c set when
 // channel c is filtered (the others pass through unchanged).
 struct IirCoefs {
