@@ -35,9 +35,9 @@ void ensure_smem(const void* kernel, int bytes);
 // The driver's unique id of the current CUDA context; 0 when none is current or the driver cannot say.
 unsigned long long current_context_id();
 
-// Tier downscale: the vertical prefilter src -> dst (same size), then the horizontal prefilter at the
-// bilinear sample points fused with the blend, v (in_w x in_h) -> dst (out_w x out_h).
-void tier_blur_v(const float* src, float* dst, const TierBlurArgs& a, cudaStream_t s);
+// Tier downscale: the vertical prefilter at the rows a.yi names, src -> dst (2 out_h rows of w pixels), then
+// the horizontal prefilter at the bilinear sample points fused with the blend -> dst (out_w x out_h).
+void tier_rows(const float* src, float* dst, const TierBlurArgs& a, cudaStream_t s);
 void tier_resample(const float* v, float* dst, const TierResampleArgs& a, cudaStream_t s);
 // Input transfer decode and geometry: src (src_w x src_h) -> dst (dst_w x dst_h).
 void prepare(const float* src, float* dst, const PrepareArgs& a, cudaStream_t s);

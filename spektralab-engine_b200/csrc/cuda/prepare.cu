@@ -4,9 +4,9 @@
 // Tier downscale (reference src/session/tiers.cpp:137-183 and kernels/session.metal:19-91): a vertical
 // Gaussian prefilter, a horizontal one, then a bilinear sample from exact-integer index tables, all in
 // binary32 with explicit fused multiply-adds in ascending tap order (so the bits do not depend on how a
-// compiler contracts). Here the vertical pass runs over the frame and the horizontal pass is evaluated
-// only at the four points each output pixel's bilinear sample reads, fused with the blend: the same
-// values as the reference's full-resolution horizontal pass, without writing and re-reading it.
+// compiler contracts). Here the vertical pass runs only at the two rows, and the horizontal pass only at the
+// four points, that an output pixel's bilinear sample reads, the latter fused with the blend: the same
+// values as the reference's full-resolution passes.
 //
 // Decode + geometry (reference kernels/film.metal:104-173): the transfer function per element, then the
 // bilinear resample at a double-float source coordinate. Both run in one pass over the output; each of
@@ -32,27 +32,67 @@ __device__ __forceinline__ int mirror_index(int i, int n) {
     return m < n ? m : period - m;
 }
 
-__global__ void k_tier_blur_v(const float* __restrict__ src, float* __restrict__ dst,
-                              const __grid_constant__ TierBlurArgs a) {
+// The vertical prefilter at rows y0 = yi[2 oy] and y1 = yi[2 oy + 1] (y0 + 1, or y0 at the bottom edge): V
+// neighbouring floats of both rows per thread, the rows they share read once, kTierTurn output rows in turn so
+// that the next row's samples are still in L1. The whole-frame form (every source row, 2 r + 1 reads per
+// value) took 0.505 ms for 6000 x 4000 to 1600 x 1066, this 0.116.
+constexpr uint32_t kTierThreads = 128, kTierTurn = 4;
+
+template <int V>
+__global__ void __launch_bounds__(kTierThreads) k_tier_rows(const float* __restrict__ src, float* __restrict__ dst,
+                                                            const __grid_constant__ TierBlurArgs a) {
     extern __shared__ float taps[];
-    const int r = a.r;
-    for (int i = threadIdx.y * blockDim.x + threadIdx.x; i <= 2 * r; i += blockDim.x * blockDim.y) taps[i] = a.taps[i];
+    const int r = a.r, h = int(a.h);
+    for (int i = threadIdx.x; i <= 2 * r; i += kTierThreads) taps[i] = a.taps[i];
     __syncthreads();
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= a.w || y >= a.h) return;
-    float acc0 = 0.0f, acc1 = 0.0f, acc2 = 0.0f;
-    for (int k = -r; k <= r; ++k) {
-        const int yy = mirror_index(int(y) + k, int(a.h));
-        const float wk = taps[k + r];
-        const float* p = src + 3 * (size_t(yy) * a.w + x);
-        acc0 = __fmaf_rn(wk, p[0], acc0);
-        acc1 = __fmaf_rn(wk, p[1], acc1);
-        acc2 = __fmaf_rn(wk, p[2], acc2);
+    const uint32_t n3 = 3 * a.w, f = V * (blockIdx.x * kTierThreads + threadIdx.x);
+    if (f >= n3) return;
+    for (uint32_t oy = blockIdx.y * kTierTurn; oy < min((blockIdx.y + 1) * kTierTurn, a.out_h); ++oy) {
+        const int y0 = int(__ldg(a.yi + 2 * oy));
+        const bool inner = y0 - r >= 0 && y0 + r + 1 < h;
+        float acc0[V], acc1[V], p[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc0[e] = acc1[e] = 0.0f;
+        const auto load = [&](int y) {
+            const float* at = src + size_t(inner ? y : mirror_index(y, h)) * n3 + f;
+            if (V == 4) {
+                const float4 t = __ldg(reinterpret_cast<const float4*>(at));
+                p[0] = t.x;
+                p[1 % V] = t.y;
+                p[2 % V] = t.z;
+                p[3 % V] = t.w;
+            } else {
+                p[0] = __ldg(at);
+            }
+        };
+        load(y0 - r);
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc0[e] = __fmaf_rn(taps[0], p[e], 0.0f);
+#pragma unroll 4
+        for (int k = 1; k <= 2 * r; ++k) {
+            load(y0 - r + k);
+            const float w0 = taps[k], w1 = taps[k - 1];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                acc0[e] = __fmaf_rn(w0, p[e], acc0[e]);
+                acc1[e] = __fmaf_rn(w1, p[e], acc1[e]);
+            }
+        }
+        load(y0 + r + 1);
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc1[e] = __fmaf_rn(taps[2 * r], p[e], acc1[e]);
+        const bool same_row = __ldg(a.yi + 2 * oy + 1) == uint32_t(y0);
+        float* q = dst + size_t(2 * oy) * n3 + f;
+        if (V == 4) {
+            const float4 t0 = make_float4(acc0[0], acc0[1 % V], acc0[2 % V], acc0[3 % V]);
+            const float4 t1 = make_float4(acc1[0], acc1[1 % V], acc1[2 % V], acc1[3 % V]);
+            *reinterpret_cast<float4*>(q) = t0;
+            *reinterpret_cast<float4*>(q + n3) = same_row ? t0 : t1;
+        } else {
+            q[0] = acc0[0];
+            q[n3] = same_row ? acc0[0] : acc1[0];
+        }
     }
-    float* q = dst + 3 * (size_t(y) * a.w + x);
-    q[0] = acc0;
-    q[1] = acc1;
-    q[2] = acc2;
 }
 
 // the horizontal prefilter of plane v (in_w wide) at (x, y)
@@ -89,7 +129,7 @@ __global__ void k_tier_resample(const float* __restrict__ v, float* __restrict__
     const uint32_t ox = blockIdx.x * blockDim.x + threadIdx.x, oy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ox >= a.out_w || oy >= a.out_h) return;
     const uint32_t x0 = a.xi[2 * ox], x1 = a.xi[2 * ox + 1];
-    const uint32_t y0 = a.yi[2 * oy], y1 = a.yi[2 * oy + 1];
+    const uint32_t y0 = a.yi ? a.yi[2 * oy] : 2 * oy, y1 = a.yi ? a.yi[2 * oy + 1] : 2 * oy + 1;
     const float tx = a.xt[ox], ty = a.yt[oy];
     float pa[3], pb[3], pd[3], pe[3];
     blur_h_at(v, taps, rx, a.in_w, x0, y0, pa);
@@ -244,12 +284,14 @@ __global__ void k_prepare(const float* __restrict__ src, float* __restrict__ dst
 
 }  // namespace
 
-void tier_blur_v(const float* src, float* dst, const TierBlurArgs& a, cudaStream_t s) {
-    const dim3 b(32, 8), g(div_up(a.w, 32), div_up(a.h, 8));
+void tier_rows(const float* src, float* dst, const TierBlurArgs& a, cudaStream_t s) {
+    const bool vec = (a.w & 3u) == 0;  // rows of whole float4
     const int smem = int((2 * a.r + 1) * sizeof(float));
-    ensure_smem(reinterpret_cast<const void*>(k_tier_blur_v), smem);
-    Probe p("tier_blur_v", s);
-    k_tier_blur_v<<<g, b, smem, s>>>(src, dst, a);
+    const dim3 g(div_up(3 * size_t(a.w), (vec ? 4 : 1) * kTierThreads), div_up(a.out_h, kTierTurn));
+    ensure_smem(vec ? reinterpret_cast<const void*>(k_tier_rows<4>) : reinterpret_cast<const void*>(k_tier_rows<1>), smem);
+    Probe p("tier_rows", s);
+    if (vec) k_tier_rows<4><<<g, kTierThreads, smem, s>>>(src, dst, a);
+    else k_tier_rows<1><<<g, kTierThreads, smem, s>>>(src, dst, a);
 }
 
 void tier_resample(const float* v, float* dst, const TierResampleArgs& a, cudaStream_t s) {

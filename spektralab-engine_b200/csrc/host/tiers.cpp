@@ -69,26 +69,24 @@ Plane downscale(Pool& pool, cudaStream_t s, const Plane& src, uint32_t long_edge
     cuda_check(cudaMemcpyAsync(tab.ptr(), words.data(), words.size() * 4, cudaMemcpyHostToDevice, s), "tier tables");
     const uint32_t* base = tab.as<uint32_t>();
 
+    const uint32_t* yi = base + oyi;
     Plane v = src;
-    Plane vb;
-    if (ty.size() > 1) {
-        vb = make_plane(pool, src.w, src.h);
-        TierBlurArgs a{reinterpret_cast<const float*>(base + oty), src.w, src.h, int32_t(ty.size() / 2)};
-        dev::tier_blur_v(src.data(), vb.data(), a, s);
-        v = vb;
+    if (ty.size() > 1) {  // the vertically filtered rows that the samples read, in the samples' order
+        v = make_plane(pool, src.w, 2 * o.h);
+        TierBlurArgs a{reinterpret_cast<const float*>(base + oty), yi, src.w, src.h, o.h, int32_t(ty.size() / 2)};
+        dev::tier_rows(src.data(), v.data(), a, s);
+        yi = nullptr;
     }
-    Plane out;
-    out.w = o.w;
-    out.h = o.h;
-    out.buf = pool.persistent(size_t(o.w) * o.h * 3 * sizeof(float));
+    // from the session's stream-ordered pool, as the frame itself: cudaMalloc and cudaFree would stop the device
+    // in every open and close
+    Plane out = make_plane(pool, o.w, o.h);
     TierResampleArgs r{};
     r.taps_x = reinterpret_cast<const float*>(base + otx);
     r.xi = base + oxi;
     r.xt = reinterpret_cast<const float*>(base + oxt);
-    r.yi = base + oyi;
+    r.yi = yi;
     r.yt = reinterpret_cast<const float*>(base + oyt);
     r.in_w = src.w;
-    r.in_h = src.h;
     r.out_w = o.w;
     r.out_h = o.h;
     r.rx = int32_t(tx.size() / 2);

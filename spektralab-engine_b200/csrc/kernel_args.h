@@ -122,21 +122,23 @@ struct CouplerArgs {
 };
 
 // Tier downscale (reference src/session/tiers.cpp:137-183, kernels/session.metal:19-91): a vertical
-// Gaussian prefilter over the frame (k_tier_blur_v), then one pass per output pixel that evaluates the
-// horizontal prefilter at the four points its bilinear sample reads and blends them. Mirror edges,
-// taps -r..r ascending, acc = fma(w_k, x, acc) from 0; the index tables are the host's exact integers.
+// Gaussian prefilter at the source rows that the bilinear sample reads (k_tier_rows: two per output row),
+// then one pass per output pixel that evaluates the horizontal prefilter at the four points its sample
+// reads and blends them. Mirror edges, taps -r..r ascending, acc = fma(w_k, x, acc) from 0; the index tables
+// are the host's exact integers.
 struct TierBlurArgs {
-    const float* taps;  // 2 r + 1
-    uint32_t w, h;
-    int32_t r;          // >= 1
+    const float* taps;   // 2 r + 1
+    const uint32_t* yi;  // [2 out_h]: i0, i1
+    uint32_t w, h, out_h;
+    int32_t r;           // >= 1
 };
 struct TierResampleArgs {
     const float* taps_x;  // 2 rx + 1 (rx = 0: no horizontal prefilter)
     const uint32_t* xi;   // [2 out_w]: i0, i1
     const float* xt;      // [out_w]
-    const uint32_t* yi;   // [2 out_h]
+    const uint32_t* yi;   // [2 out_h]; null: the rows are k_tier_rows' (2 oy, 2 oy + 1)
     const float* yt;      // [out_h]
-    uint32_t in_w, in_h, out_w, out_h;
+    uint32_t in_w, out_w, out_h;
     int32_t rx;
 };
 
@@ -173,6 +175,7 @@ struct MeterSelect {
     uint64_t prefix[kMeterQueries];  // the ordered key's digits found so far
     uint64_t mask[kMeterQueries];
     uint32_t hist[kMeterQueries][256];
+    uint32_t blocks_done;            // of the current digit's histogram launch
     double value[kMeterQueries];     // the selected luminances
 };
 struct MeterOut {
