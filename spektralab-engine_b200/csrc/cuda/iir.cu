@@ -25,9 +25,11 @@
 //             of 4 pixels, is a 2-D tensor (3 pitch floats x h rows), and the strip is a column of 12-float
 //             boxes of up to 256 rows, all completing on one mbarrier.
 //             Column pass, the sum in a global plane and scalar copies at odd widths before: 3840 x 2160, two
-//             components 0.289 -> 0.259 ms; 6000 x 4000, three 1.70 -> 1.31; 1999 x 1333, three 0.339 -> 0.143.
-//             At 6000 x 4000 the loads take 0.29 ms of it, raw 0.28, the recurrences the rest (one strip of
-//             twelve warps per SM; the 32-to-64-bit conversions' unit is the busiest in that phase). Its waits are bounded: one that gives up counts
+//             components 0.290 -> 0.239 ms; 6000 x 4000, two 1.06 -> 0.88; 1999 x 1333, two 0.219 -> 0.100.
+//             With three components at 6000 x 4000 the loads take 0.29 ms, raw 0.28, the recurrences the rest
+//             (one strip of twelve warps per SM; the 32-to-64-bit conversions' unit is the busiest there).
+//             Loading and converting eight samples ahead of their chain made the recurrences slower (0.88 ->
+//             1.09 ms; rows at 4K 0.150 -> 0.187): the unrolled loop already overlaps them. Its waits are bounded: one that gives up counts
 //             itself (g_iir_gave_up), waits again under the full limit for the copies in flight, and if
 //             even they never land the CTA loads this and every later strip with plain copies.
 #include <cuda.h>
@@ -58,7 +60,7 @@ constexpr int kColLines = 3 * kColPixels;
 constexpr int kSegCols = SPKB_IIR_SEG_COLS;  // segments per column line (32: two 4K strips per SM)
 static_assert(kSegCols <= (1 << kIirScanSteps), "the carry scan composes at most 2^kIirScanSteps segments");
 constexpr int kColThreads = kColLines * kSegCols;
-constexpr int kColBlocks = 2;  // resident strips the register allocation allows (a 4K column pass holds two)
+
 
 // The column pass's tensor maps, one per component plane, and the strip's box geometry: `boxes` boxes of
 // `box_rows` rows (a multiple of 8, at most 256) cover the frame's rows; the strip buffer holds
@@ -153,9 +155,7 @@ struct Coef {
 // it enters the j-th multiply-add from the end, so the chain costs one multiply-add latency per sample.
 // One pass over the segment [a, b) of a line in shared memory (element i at base[i * stride]), ascending or
 // descending. Zero-state run: returns the end state. Writing run: from the state given, stores float(w)
-// back. Samples go in chunks of kRunChunk, loaded, converted and scaled ahead of the chain, so that a step
-// waits for the one multiply-add that takes the newest state.
-constexpr int kRunChunk = 8;
+// back.
 
 template <bool FORWARD, bool WRITE>
 __device__ __forceinline__ void seg_run(const Coef& k, float* base, int stride, int a, int b, double& s1, double& s2,
@@ -169,20 +169,8 @@ __device__ __forceinline__ void seg_run(const Coef& k, float* base, int stride, 
         s1 = t;
         return float(t);
     };
-    int i = 0;
-#pragma unroll 1
-    for (; i + kRunChunk <= n; i += kRunChunk, p += kRunChunk * dir) {
-        double kx[kRunChunk];
-#pragma unroll
-        for (int j = 0; j < kRunChunk; ++j) kx[j] = k.B * double(p[j * dir]);
-#pragma unroll
-        for (int j = 0; j < kRunChunk; ++j) {
-            const float v = chain(kx[j]);
-            if (WRITE) p[j * dir] = v;
-        }
-    }
-#pragma unroll 1
-    for (; i < n; ++i, p += dir) {
+#pragma unroll 4
+    for (int i = 0; i < n; ++i, p += dir) {
         const float v = chain(k.B * double(*p));
         if (WRITE) *p = v;
     }
@@ -407,8 +395,9 @@ __device__ __forceinline__ QuadWeights quad_weights(const float (&w)[3]) {
     const int j = 4 * (int(threadIdx.x) % kQuads);
     return {{w[j % 3], w[(j + 1) % 3], w[(j + 2) % 3], w[j % 3]}};
 }
+template <bool MULTI>
 __device__ __forceinline__ float4 sum_quad(const QuadWeights& wc, const float4& v, bool first, uint32_t taddr) {
-    if (first) return make_float4(0.0f + wc.w[0] * v.x, 0.0f + wc.w[1] * v.y, 0.0f + wc.w[2] * v.z, 0.0f + wc.w[3] * v.w);
+    if (!MULTI || first) return make_float4(0.0f + wc.w[0] * v.x, 0.0f + wc.w[1] * v.y, 0.0f + wc.w[2] * v.z, 0.0f + wc.w[3] * v.w);
     const float4 a = tmem_ld4(taddr);
     return make_float4(a.x + wc.w[0] * v.x, a.y + wc.w[1] * v.y, a.z + wc.w[2] * v.z, a.w + wc.w[3] * v.w);
 }
@@ -421,23 +410,26 @@ __device__ __forceinline__ float mix2(float mx, float x, float my, float y) { re
 // The blurred strip of component c joins the sum: acc := 0 + w v or acc + w v. The result goes back to the
 // tensor memory, or (to_strip) over the strip. Every lane of a warp with a quad left takes part in the
 // tensor-memory accesses; the quads past the frame's rows are the strip buffer's padding or its last row.
+template <bool MULTI>
 __device__ __forceinline__ void strip_sum(float* strip, int n, const IirMixture& mix, int c, uint32_t tmem, bool to_strip) {
     const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads, last = n - 1;
     const QuadWeights wc = quad_weights(mix.weight[c]);
     uint32_t taddr = tmem + (uint32_t(32 * (warp & 3)) << 16) + 4u * uint32_t(warp >> 2);
     for (int q0 = 32 * warp, row = int(threadIdx.x) / kQuads; q0 < kQuads * n; q0 += kColThreads, row += kQuadRows, taddr += 12u) {
         float4* at = reinterpret_cast<float4*>(strip + size_t(min(row, last)) * kColLines + 4 * qd);
-        const float4 a = sum_quad(wc, *at, c == 0, taddr);
-        if (!to_strip) tmem_st4(taddr, a);
+        const float4 a = sum_quad<MULTI>(wc, *at, c == 0, taddr);
+        if (MULTI && !to_strip) tmem_st4(taddr, a);
         else if (row <= last) *at = a;
     }
-    if (!to_strip) tmem_wait_st();
+    if (MULTI && !to_strip) tmem_wait_st();
 }
 
 // raw := mix_a raw + mix_b (the sum after the last component c), or the strip as it is (plain), in float4.
-// A thread steps down the rows kStoreBatch at a time, their reads issued before the first store.
-constexpr int kStoreBatch = 4;
+// A thread steps down the rows kStoreBatch at a time, their reads issued before the first store (4K 0.239 ms at
+// one and two, 0.258 at four; 6000 x 4000 0.93, 0.88, 0.87).
+constexpr int kStoreBatch = 2;
 
+template <bool MULTI>
 __device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, size_t pitch, int n, const IirMixture& mix,
                                              int c, uint32_t tmem) {
     const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads;
@@ -460,7 +452,7 @@ __device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, siz
             const int r = min(row, n - 1);
             float4 v = *reinterpret_cast<const float4*>(strip + size_t(r) * kColLines + 4 * qd);
             if (!plain) {
-                const float4 a = sum_quad(wc, v, c == 0, taddr);
+                const float4 a = sum_quad<MULTI>(wc, v, c == 0, taddr);
                 v.x = mix2(ma.w[0], rw[u].x, mb.w[0], a.x);
                 v.y = mix2(ma.w[1], rw[u].y, mb.w[1], a.y);
                 v.z = mix2(ma.w[2], rw[u].z, mb.w[2], a.z);
@@ -499,7 +491,11 @@ __device__ __forceinline__ void strip_to_raw_scalar(const float* strip, float* r
     }
 }
 
-__global__ void __launch_bounds__(kColThreads, kColBlocks) k_iir_cols(float* raw, const __grid_constant__ IirPlanes hs, uint32_t w, uint32_t h,
+// MULTI: more than one component, the sum in tensor memory. Registers for two strips per SM (what shared
+// memory holds at 4K): held to three or four, even short frames ran slower (1024 x 1024, one component: 0.030 ms
+// at two, 0.035 and 0.038).
+template <bool MULTI>
+__global__ void __launch_bounds__(kColThreads, 2) k_iir_cols(float* raw, const __grid_constant__ IirPlanes hs, uint32_t w, uint32_t h,
                                                           const __grid_constant__ IirMixture mix,
                                                           const __grid_constant__ IirColMaps maps) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -527,7 +523,7 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_iir_cols(float* raw
     }
     const uint32_t tmem_slot = bar + 8;
     uint32_t tmem = 0;
-    if (maps.tmem_cols != 0) {
+    if (MULTI) {
         if (threadIdx.x < 32) {
             tmem_alloc(tmem_slot, maps.tmem_cols);
             tmem_relinquish();
@@ -575,20 +571,20 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks) k_iir_cols(float* raw
         }
         __syncthreads();
         blur_lines(strip, kColLines, kColLines, n, kSegCols, mix.cols, c, carry, false);
-        if (mix.plain == 0 && c + 1 < int(mix.ncomp)) {
-            strip_sum(strip, n, mix, c, tmem, false);
+        if (MULTI && c + 1 < int(mix.ncomp)) {
+            strip_sum<MULTI>(strip, n, mix, c, tmem, false);
         } else if (raw_vec) {
-            strip_to_raw(strip, raw + off, raw_pitch, n, mix, c, tmem);
+            strip_to_raw<MULTI>(strip, raw + off, raw_pitch, n, mix, c, tmem);
         } else {
             if (mix.plain == 0) {
-                strip_sum(strip, n, mix, c, tmem, true);
+                strip_sum<MULTI>(strip, n, mix, c, tmem, true);
                 __syncthreads();
             }
             strip_to_raw_scalar(strip, raw + off, raw_pitch, nl, n, mix);
         }
         __syncthreads();
     }
-    if (maps.tmem_cols != 0) {
+    if (MULTI) {
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
@@ -728,10 +724,12 @@ void iir_mixture(const float* src, float* raw, float* const* tmp, uint32_t w, ui
     for (uint32_t c = 0; c < m.ncomp; ++c) planes.p[c] = tmp[c];
     const size_t sr = iir_rows_smem(m.pitch), sc = iir_cols_smem(h);
     ensure_smem(reinterpret_cast<const void*>(k_iir_rows), int(sr));
-    ensure_smem(reinterpret_cast<const void*>(k_iir_cols), int(sc));
+    const bool multi = m.ncomp > 1;
+    ensure_smem(multi ? reinterpret_cast<const void*>(k_iir_cols<true>) : reinterpret_cast<const void*>(k_iir_cols<false>),
+                int(sc));
     IirColMaps maps{};
     col_maps(maps, planes, m.ncomp, m.pitch, h);
-    if (m.ncomp > 1) {
+    if (multi) {
         // four columns for every 128 quads; allocations are powers of two from 32
         const uint32_t need = 4u * ((3u * h + 127u) / 128u);
         maps.tmem_cols = 32;
@@ -743,7 +741,9 @@ void iir_mixture(const float* src, float* raw, float* const* tmp, uint32_t w, ui
     }
     {
         Probe p("iir_cols", s);
-        k_iir_cols<<<(w + kColPixels - 1) / kColPixels, kColThreads, sc, s>>>(raw, planes, w, h, m, maps);
+        const uint32_t g = (w + kColPixels - 1) / kColPixels;
+        if (multi) k_iir_cols<true><<<g, kColThreads, sc, s>>>(raw, planes, w, h, m, maps);
+        else k_iir_cols<false><<<g, kColThreads, sc, s>>>(raw, planes, w, h, m, maps);
     }
 }
 
