@@ -2446,14 +2446,43 @@ SPK_API spk_status spk_render_vjp(spk_session* session, const char* tier, uint32
         if (grad_output) {
             dgy = s.pool.acquire(bytes);
             dgx = s.pool.acquire(bytes);
-            cuda_check(cudaMemcpyAsync(dgy.ptr(), grad_output, bytes, cudaMemcpyHostToDevice, s.stream), "copy");
         }
-        render_vjp(ctx, s.pipe, s.live, s.source, film_seed, s.hal, output ? dy.as<float>() : nullptr,
-                   grad_output ? dgy.as<float>() : nullptr, grad_output ? dgx.as<float>() : nullptr,
-                   grad_output ? grad_params : nullptr, grad_output ? n_params : 0u);
-        if (output) cuda_check(cudaMemcpyAsync(output, dy.ptr(), bytes, cudaMemcpyDeviceToHost, s.stream), "copy");
+        // The copies of pageable host arrays hold this thread: the upstream gradient goes up while the device
+        // runs the forward, the output comes down while it runs the adjoint, both on the copy stream.
+        std::vector<cudaEvent_t>& ev = s.band_events;
+        while (ev.size() < 2) {
+            cudaEvent_t e = nullptr;
+            cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "adjoint event");
+            ev.push_back(e);
+        }
+        struct CopyGuard {  // no copy is under way when the buffers go
+            cudaStream_t c;
+            ~CopyGuard() { (void)cudaStreamSynchronize(c); }
+        } copies{s.copy_stream};
+        // the buffers are the copy stream's to use from here on
+        cuda_check(cudaEventRecord(ev[0], s.stream), "adjoint event");
+        cuda_check(cudaStreamWaitEvent(s.copy_stream, ev[0], 0), "adjoint event");
+        render_vjp(
+            ctx, s.pipe, s.live, s.source, film_seed, s.hal, output ? dy.as<float>() : nullptr,
+            grad_output ? dgy.as<float>() : nullptr, grad_output ? dgx.as<float>() : nullptr,
+            grad_output ? grad_params : nullptr, grad_output ? n_params : 0u,
+            [&] {
+                cuda_check(cudaEventRecord(ev[0], s.stream), "adjoint event");  // y is written
+                if (!grad_output) return;
+                cuda_check(cudaMemcpyAsync(dgy.ptr(), grad_output, bytes, cudaMemcpyHostToDevice, s.copy_stream), "copy");
+                cuda_check(cudaEventRecord(ev[1], s.copy_stream), "adjoint event");
+                cuda_check(cudaStreamWaitEvent(s.stream, ev[1], 0), "adjoint event");
+            },
+            [&] {
+                if (!output) return;
+                cuda_check(cudaStreamWaitEvent(s.copy_stream, ev[0], 0), "adjoint event");
+                cuda_check(cudaMemcpyAsync(output, dy.ptr(), bytes, cudaMemcpyDeviceToHost, s.copy_stream), "copy");
+            });
+        if (output && !grad_output)
+            cuda_check(cudaMemcpyAsync(output, dy.ptr(), bytes, cudaMemcpyDeviceToHost, s.stream), "copy");
         if (grad_output)
             cuda_check(cudaMemcpyAsync(grad_input, dgx.ptr(), bytes, cudaMemcpyDeviceToHost, s.stream), "copy");
+        cuda_check(cudaStreamSynchronize(s.copy_stream), "render adjoint");
         cuda_check(cudaStreamSynchronize(s.stream), "render adjoint");
         cuda_check(cudaGetLastError(), "render adjoint");
         return SPK_OK;

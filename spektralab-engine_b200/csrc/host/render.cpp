@@ -1330,7 +1330,8 @@ dev::VjpPrintArgs vjp_print_args(const Pipeline& p, const LiveParams& live, uint
 
 void render_vjp(RenderCtx& ctx, const Pipeline& p, const LiveParams& live, const Plane& source, uint32_t film_seed,
                 const std::optional<HalationOverride>& hov, float* y_out, const float* g_y, float* g_x,
-                double* grad_params, uint32_t n_params) {
+                double* grad_params, uint32_t n_params, const std::function<void()>& forward_enqueued,
+                const std::function<void()>& adjoint_enqueued) {
     const FilmSetup& f = *p.film;
     const PrintSetup& ps = *p.print;
     const uint32_t w = source.w, h = source.h;
@@ -1418,6 +1419,7 @@ void render_vjp(RenderCtx& ctx, const Pipeline& p, const LiveParams& live, const
         lincomb(ctx, Vec3{1.0 + am, 1.0 + am, 1.0 + am}, B, Vec3{-am, -am, -am}, &Gs, Y);
     }
     if (y_out) cuda_check(cudaMemcpyAsync(y_out, Y.data(), Y.bytes(), cudaMemcpyDeviceToDevice, ctx.stream), "copy");
+    forward_enqueued();
     if (!g_y) return;
 
     // ---- adjoint ----
@@ -1460,6 +1462,7 @@ void render_vjp(RenderCtx& ctx, const Pipeline& p, const LiveParams& live, const
     if (pl.scatter) mixture_adjoint(ctx, g, pl.scatter_comps, pl.scatter_a, pl.scatter_b);  // g_H1
     if (s_lens > 0.0) gaussian_adjoint(ctx, g, s_lens);  // g_H0
     dev::vjp_expose(source.data(), g.data(), g_x, p.dev.table.as<float>(), ea, ctx.stream);
+    adjoint_enqueued();
     double hp[kAcc];
     cuda_check(cudaMemcpyAsync(hp, dparams.ptr(), sizeof hp, cudaMemcpyDeviceToHost, ctx.stream), "copy");
     cuda_check(cudaStreamSynchronize(ctx.stream), "render adjoint");

@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <optional>
 #include <vector>
 
@@ -139,9 +140,13 @@ void print_nodes(RenderCtx& ctx, const PrintSetup& s);
 //    density-curve parameter (layer c, node j) at 3 + 2K + 16 c + j],
 // K the components of the halation override (none without one). A weight's or sigma's gradient is along
 // a common change of its three channels; the curve parameters are the hat functions of vjp.hpp.
+// forward_enqueued is called once the forward's work (y_out written) is on ctx.stream and must have the
+// stream wait for g_y; adjoint_enqueued once all of the adjoint's is, before the call waits for it: host
+// copies made there overlap the device's work.
 void render_vjp(RenderCtx& ctx, const Pipeline& p, const LiveParams& live, const Plane& source, uint32_t film_seed,
                 const std::optional<HalationOverride>& hov, float* y_out, const float* g_y, float* g_x,
-                double* grad_params, uint32_t n_params);
+                double* grad_params, uint32_t n_params, const std::function<void()>& forward_enqueued,
+                const std::function<void()>& adjoint_enqueued);
 
 // The DIR-coupler diffusion (reference src/fx/dir_blur.hpp:15-19, dir_blur.cpp:14-38) at a pixel pitch: a
 // core Gaussian of 20 um with weight 1 - 0.06 and the exponential surrogate of a 200 um tail with weight 0.06.
