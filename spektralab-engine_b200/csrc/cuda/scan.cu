@@ -19,6 +19,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../kernel_args.h"
 #include "encode.cuh"
 #include "launch.hpp"
@@ -36,6 +38,82 @@ static_assert(uint32_t(kTH) == scan_tile_rows(), "row bands start on tile rows")
 
 // half-sample symmetric reflection, exact for p in [-n, 2n)
 __device__ __forceinline__ int reflect_near(int p, int n) { return p < 0 ? -1 - p : (p >= n ? 2 * n - 1 - p : p); }
+
+// FIR passes over rows in shared memory with register windows: a thread forms kWin outputs of one float
+// column (window_v) or of one channel in one row (window_h) and reads each input they share once; every output
+// is sum_k t[k] x[i + k] from 0, k ascending. window_v: rows x cols floats of dst from rows + 2 R of src;
+// window_h: rows x px pixels of dst from px + 2 R of src. Outputs past the image are formed from whatever
+// the rows hold and never used.
+// 12 outputs: the 36 rows and pixels of the 4K scanner's lens-blurred tile take three windows each, one turn
+// of the CTA (4K scanner 0.185 ms with 6 and 4, two turns, 0.172 with 12).
+constexpr int kWin = 12;
+
+template <int R>
+__device__ __forceinline__ void window_v(const float* src, int sp, float* dst, int dp, int rows, int cols, const float* t) {
+    constexpr int T = 2 * R + 1;
+    const int items = cols * ((rows + kWin - 1) / kWin);
+    for (int item = threadIdx.x; item < items; item += kThreads) {
+        const int blk = item / cols, f = item - blk * cols, i0 = blk * kWin;
+        float acc[kWin];
+#pragma unroll
+        for (int o = 0; o < kWin; ++o) acc[o] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kWin + T - 1; ++j)
+            if (i0 + j < rows + T - 1) {
+                const float v = src[(i0 + j) * sp + f];
+#pragma unroll
+                for (int o = 0; o < kWin; ++o)
+                    if (j - o >= 0 && j - o < T) acc[o] += t[j - o] * v;
+            }
+#pragma unroll
+        for (int o = 0; o < kWin; ++o)
+            if (i0 + o < rows) dst[(i0 + o) * dp + f] = acc[o];
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void window_h(const float* src, int sp, float* dst, int dp, int rows, int px, const float* t) {
+    constexpr int T = 2 * R + 1;
+    const int per = 3 * ((px + kWin - 1) / kWin), items = rows * per;
+    for (int item = threadIdx.x; item < items; item += kThreads) {
+        const int i = item / per, rem = item - i * per, c = rem % 3, j0 = (rem / 3) * kWin;
+        const float* row = src + i * sp + c;
+        float acc[kWin];
+#pragma unroll
+        for (int o = 0; o < kWin; ++o) acc[o] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kWin + T - 1; ++q)
+            if (j0 + q < px + T - 1) {
+                const float v = row[3 * (j0 + q)];
+#pragma unroll
+                for (int o = 0; o < kWin; ++o)
+                    if (q - o >= 0 && q - o < T) acc[o] += t[q - o] * v;
+            }
+#pragma unroll
+        for (int o = 0; o < kWin; ++o)
+            if (j0 + o < px) dst[i * dp + 3 * (j0 + o) + c] = acc[o];
+    }
+}
+
+// f<R>() for the radius r, 1 .. SPKB_FIR_MAX_R; RC >= 0: r is RC, known when compiled
+template <int RC, class F>
+__device__ __forceinline__ void with_radius(int r, F&& f) {
+    if constexpr (RC >= 0) {
+        f(std::integral_constant<int, RC>());
+    } else {
+        switch (r) {
+            case 1: f(std::integral_constant<int, 1>()); break;
+            case 2: f(std::integral_constant<int, 2>()); break;
+            case 3: f(std::integral_constant<int, 3>()); break;
+            case 4: f(std::integral_constant<int, 4>()); break;
+            case 5: f(std::integral_constant<int, 5>()); break;
+            case 6: f(std::integral_constant<int, 6>()); break;
+            case 7: f(std::integral_constant<int, 7>()); break;
+            case 8: f(std::integral_constant<int, 8>()); break;
+            default: f(std::integral_constant<int, 9>()); break;
+        }
+    }
+}
 
 // One 32 x 32 output tile at (x0, y0) of a frame; smem as sized by scan_smem_bytes for the radii.
 template <int R1, int R2>
@@ -70,97 +148,13 @@ __device__ __forceinline__ void scan_tile(const ScanArgs& a, const float* __rest
     }
     __syncthreads();
 
-    if constexpr (R1 >= 0 && R2 >= 0) {
-        // 2. lens blur, vertical, with register windows: a thread takes kVRows consecutive output rows of
-        //    one column and reads each input row once; every output is still sum_k t1[k] A[i + k] from 0,
-        //    k ascending
-        constexpr int T1 = 2 * R1 + 1, PCc = 3 * (kTW + 2 * (R1 + R2)), PRc = kTH + 2 * (R1 + R2);
-        constexpr int BRc = kTH + 2 * R2, BCc = 3 * (kTW + 2 * R2);
-        constexpr int kVRows = 6, NB = (BRc + kVRows - 1) / kVRows;
-        for (int item = threadIdx.x; item < PCc * NB; item += kThreads) {
-            const int f = item % PCc, i0 = (item / PCc) * kVRows;
-            float acc[kVRows];
-#pragma unroll
-            for (int o = 0; o < kVRows; ++o) acc[o] = 0.0f;
-#pragma unroll
-            for (int j = 0; j < kVRows + T1 - 1; ++j) {
-                if (i0 + j < PRc) {
-                    const float v = A[(i0 + j) * PCc + f];
-#pragma unroll
-                    for (int o = 0; o < kVRows; ++o)
-                        if (j - o >= 0 && j - o < T1) acc[o] += a.t1[j - o] * v;
-                }
-            }
-#pragma unroll
-            for (int o = 0; o < kVRows; ++o) {
-                const int i = i0 + o, yy = y0 - R2 + i;
-                if (i < BRc && yy >= 0 && yy < h) B[i * PCc + f] = acc[o];
-            }
-        }
+    // 2., 3. lens blur, vertical (B: the tile's rows and its r2 halo, every column) and horizontal (back to A);
+    // without one the tile as loaded is the lens-blurred tile, its rows at the same pitch
+    if (r1 > 0) {
+        with_radius<R1>(r1, [&](auto r) { window_v<decltype(r)::value>(A, PC, B, PC, BR, PC, a.t1); });
         __syncthreads();
-
-        // 3. lens blur, horizontal, with register windows: a thread takes kHPix consecutive output pixels
-        //    of one channel in one row
-        constexpr int kHPix = 4, NG = (kTW + 2 * R2 + kHPix - 1) / kHPix;
-        for (int item = threadIdx.x; item < BRc * 3 * NG; item += kThreads) {
-            const int i = item / (3 * NG), rem = item - i * (3 * NG), c = rem % 3, j0 = (rem / 3) * kHPix;
-            const int yy = y0 - R2 + i;
-            if (yy < 0 || yy >= h) continue;
-            float acc[kHPix];
-#pragma unroll
-            for (int o = 0; o < kHPix; ++o) acc[o] = 0.0f;
-            const float* brow = B + i * PCc + c;
-#pragma unroll
-            for (int q = 0; q < kHPix + T1 - 1; ++q) {
-                if (j0 + q < kTW + 2 * (R1 + R2)) {
-                    const float v = brow[3 * (j0 + q)];
-#pragma unroll
-                    for (int o = 0; o < kHPix; ++o)
-                        if (q - o >= 0 && q - o < T1) acc[o] += a.t1[q - o] * v;
-                }
-            }
-#pragma unroll
-            for (int o = 0; o < kHPix; ++o) {
-                const int jb = j0 + o;
-                if (jb >= kTW + 2 * R2) break;
-                if (!inner_x) {
-                    const int xx = x0 - R2 + jb;
-                    if (xx < 0 || xx >= w) continue;
-                }
-                A[i * BCc + 3 * jb + c] = acc[o];
-            }
-        }
+        with_radius<R1>(r1, [&](auto r) { window_h<decltype(r)::value>(B, PC, A, BC, BR, kTW + 2 * r2, a.t1); });
         __syncthreads();
-    } else {
-    // 2. lens blur, vertical: rows y0 - r2 + i inside the image, every column of the tile
-    for (int i = warp; i < BR; i += kWarps) {
-        const int yy = y0 - r2 + i;
-        if (yy < 0 || yy >= h) continue;
-        for (int f = lane; f < PC; f += 32) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int k = 0; k <= 2 * r1; ++k) acc += a.t1[k] * A[(i + k) * PC + f];
-            B[i * PC + f] = acc;
-        }
-    }
-    __syncthreads();
-
-    // 3. lens blur, horizontal: pixels (y0 - r2 + i, x0 - r2 + jb) inside the image, into A
-    for (int i = warp; i < BR; i += kWarps) {
-        const int yy = y0 - r2 + i;
-        if (yy < 0 || yy >= h) continue;
-        for (int fb = lane; fb < BC; fb += 32) {
-            if (!inner_x) {
-                const int xx = x0 - r2 + fb / 3;
-                if (xx < 0 || xx >= w) continue;
-            }
-            float acc = 0.0f;
-#pragma unroll
-            for (int k = 0; k <= 2 * r1; ++k) acc += a.t1[k] * B[i * PC + fb + 3 * k];
-            A[i * BC + fb] = acc;
-        }
-    }
-    __syncthreads();
     }
 
     if (r2 > 0) {
@@ -182,40 +176,8 @@ __device__ __forceinline__ void scan_tile(const ScanArgs& a, const float* __rest
             }
             __syncthreads();
         }
-        // 5. unsharp blur, vertical: the tile's rows inside the image, every column of the blurred tile
-        if constexpr (R2 >= 0) {
-            // register windows of kURows rows per thread, as in step 2
-            constexpr int T2 = 2 * R2 + 1, BCc = 3 * (kTW + 2 * R2), BRc = kTH + 2 * R2;
-            constexpr int kURows = 8, NU = kTH / kURows;
-            for (int item = threadIdx.x; item < BCc * NU; item += kThreads) {
-                const int fb = item % BCc, i0 = (item / BCc) * kURows;
-                float acc[kURows];
-#pragma unroll
-                for (int o = 0; o < kURows; ++o) acc[o] = 0.0f;
-#pragma unroll
-                for (int j = 0; j < kURows + T2 - 1; ++j) {
-                    if (i0 + j < BRc) {
-                        const float v = A[(i0 + j) * BCc + fb];
-#pragma unroll
-                        for (int o = 0; o < kURows; ++o)
-                            if (j - o >= 0 && j - o < T2) acc[o] += a.t2[j - o] * v;
-                    }
-                }
-#pragma unroll
-                for (int o = 0; o < kURows; ++o)
-                    if (y0 + i0 + o < h) B[(i0 + o) * BCc + fb] = acc[o];
-            }
-        } else {
-        for (int i = warp; i < kTH; i += kWarps) {
-            if (y0 + i >= h) break;
-            for (int fb = lane; fb < BC; fb += 32) {
-                float acc = 0.0f;
-#pragma unroll
-                for (int k = 0; k <= 2 * r2; ++k) acc += a.t2[k] * A[(i + k) * BC + fb];
-                B[i * BC + fb] = acc;
-            }
-        }
-        }
+        // 5. unsharp blur, vertical, every column of the blurred tile
+        with_radius<R2>(r2, [&](auto r) { window_v<decltype(r)::value>(A, BC, B, BC, kTH, BC, a.t2); });
         __syncthreads();
     }
 
@@ -497,6 +459,21 @@ size_t scan_smem_bytes(int r1, int r2) {
     return size_t((kTH + 2 * R) + (kTH + 2 * r2)) * size_t(3 * (kTW + 2 * R)) * sizeof(float);
 }
 
+// f(R1, R2) with the radii known when compiled where they are common (-1: read from the arguments): the unsharp
+// mask's 2 px at the full tier and 1 px on the smaller ones, no lens blur, or the 5 px of a 1.5 px one. The last
+// step's unsharp sum is what a radius read at run time slows down (4K, no lens blur: 0.113 ms against 0.158).
+template <class F>
+void with_scan_radii(int r1, int r2, F&& f) {
+    const auto lens = [&](auto c2) {
+        if (r1 == 0) f(std::integral_constant<int, 0>(), c2);
+        else if (r1 == 5) f(std::integral_constant<int, 5>(), c2);
+        else f(std::integral_constant<int, -1>(), c2);
+    };
+    if (r2 == 1) lens(std::integral_constant<int, 1>());
+    else if (r2 == 2) lens(std::integral_constant<int, 2>());
+    else f(std::integral_constant<int, -1>(), std::integral_constant<int, -1>());
+}
+
 template <int R1, int R2>
 void launch_scan(const float* rgb, uint16_t* out, uint32_t w, uint32_t h, uint32_t row0, uint32_t row1,
                  const ScanArgs& a, cudaStream_t s) {
@@ -518,9 +495,9 @@ void scan_encode_rows(const float* rgb, uint16_t* out, uint32_t w, uint32_t h, u
                       const ScanArgs& a, cudaStream_t s) {
     if (uint64_t(w) * h == 0 || row1 <= row0) return;
     Probe p("scan_encode", s);
-    if (a.r1 == 5 && a.r2 == 2) launch_scan<5, 2>(rgb, out, w, h, row0, row1, a, s);
-    else if (a.r1 == 0 && a.r2 == 2) launch_scan<0, 2>(rgb, out, w, h, row0, row1, a, s);
-    else launch_scan<-1, -1>(rgb, out, w, h, row0, row1, a, s);
+    with_scan_radii(a.r1, a.r2, [&](auto r1, auto r2) {
+        launch_scan<decltype(r1)::value, decltype(r2)::value>(rgb, out, w, h, row0, row1, a, s);
+    });
 }
 
 void scan_encode(const float* rgb, uint16_t* out, uint32_t w, uint32_t h, const ScanArgs& a, cudaStream_t s) {
@@ -538,11 +515,12 @@ void launch_scan_batch(const BatchScanFrame* frames, uint32_t n_frames, uint32_t
 
 void scan_prepare() {
     const int max_smem = int(scan_smem_bytes(SPKB_FIR_MAX_R, SPKB_FIR_MAX_R));
-    ensure_smem(reinterpret_cast<const void*>(k_scan_encode<5, 2>), int(scan_smem_bytes(5, 2)));
-    ensure_smem(reinterpret_cast<const void*>(k_scan_encode<0, 2>), int(scan_smem_bytes(0, 2)));
-    ensure_smem(reinterpret_cast<const void*>(k_scan_encode<-1, -1>), max_smem);
-    ensure_smem(reinterpret_cast<const void*>(k_scan_encode_batch<5, 2>), int(scan_smem_bytes(5, 2)));
-    ensure_smem(reinterpret_cast<const void*>(k_scan_encode_batch<-1, -1>), max_smem);
+    const auto set = [&](auto r1, auto r2) {
+        ensure_smem(reinterpret_cast<const void*>(k_scan_encode<decltype(r1)::value, decltype(r2)::value>), max_smem);
+        ensure_smem(reinterpret_cast<const void*>(k_scan_encode_batch<decltype(r1)::value, decltype(r2)::value>), max_smem);
+    };
+    for (int r1 : {0, 1, 5})
+        for (int r2 : {1, 2, 3}) with_scan_radii(r1, r2, set);
 }
 
 uint32_t scan_tiles(uint32_t w, uint32_t h) { return ((w + kTW - 1) / kTW) * ((h + kTH - 1) / kTH); }
@@ -552,8 +530,10 @@ void scan_encode_batch(const BatchScanFrame* frames, uint32_t n_frames, uint32_t
                        uint32_t ctas, cudaStream_t s) {
     if (n_tiles == 0) return;
     Probe p("scan_encode_batch", s);
-    if (r1 == 5 && r2 == 2) launch_scan_batch<5, 2>(frames, n_frames, n_tiles, ctas, scan_smem_bytes(5, 2), s);
-    else launch_scan_batch<-1, -1>(frames, n_frames, n_tiles, ctas, scan_smem_bytes(SPKB_FIR_MAX_R, SPKB_FIR_MAX_R), s);
+    const size_t smem = r1 >= 0 && r2 >= 0 ? scan_smem_bytes(r1, r2) : scan_smem_bytes(SPKB_FIR_MAX_R, SPKB_FIR_MAX_R);
+    with_scan_radii(r1, r2, [&](auto c1, auto c2) {
+        launch_scan_batch<decltype(c1)::value, decltype(c2)::value>(frames, n_frames, n_tiles, ctas, smem, s);
+    });
 }
 
 namespace {
