@@ -27,7 +27,8 @@ namespace {
 
 // 512 threads per CTA: the warps of a CTA start together and run the same fully unrolled spectral code
 // close behind one another, so they share its instruction-cache lines (4K print 0.648 ms at 128 threads,
-// 0.566 at 256, 0.527 at 512, outputs identical)
+// 0.566 at 256, 0.527 at 512, outputs identical; 0.512 with the gamut stage's special-function operations in
+// their .ftz forms)
 #ifndef SPKB_PRINT_THREADS
 #define SPKB_PRINT_THREADS 512
 #endif
@@ -208,8 +209,11 @@ __global__ void __launch_bounds__(kPrintThreads) k_print_batch_shared(const Batc
 void print(const float* neg, float* rgb, const PrintArgs& a, cudaStream_t s) {
     if (a.n == 0) return;
     const uint32_t threads = (a.n + 2 * kPairs - 1) / (2 * kPairs);
+    // Fewer than two full CTAs per SM leave SMs idle or unevenly loaded: quarter-size ones spread such a print
+    // (131 x 97: 0.0259 -> 0.0225 ms, 512 x 512: 0.0335 -> 0.0316; 1600 x 256 already 0.0427 -> 0.0482)
+    const uint32_t cta = threads < 2u * 148u * kPrintThreads ? kPrintThreads / 4 : kPrintThreads;
     Probe p("print", s);
-    k_print<<<(threads + kPrintThreads - 1) / kPrintThreads, kPrintThreads, 0, s>>>(neg, rgb, a);
+    k_print<<<(threads + cta - 1) / cta, cta, 0, s>>>(neg, rgb, a);
 }
 
 void print_batch(const BatchPrintFrame* frames, const uint32_t* item_frame, const uint32_t* item_first,

@@ -52,14 +52,17 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
 
 __device__ __forceinline__ float lg2_approx(float x) {
     float y;
-    asm("lg2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// The approximate operations take their .ftz forms, one special-function instruction each: the others
+// scale subnormal operands and results around it, and no value here that is not zero is below 1e-30 (the
+// sums carry kTiny, the gamut stage works on percentages). Same results on normal numbers.
 // a / b with PTX div.approx (2 ulp for |b| in [2^-126, 2^126]); a / 0 = +-inf, 0 / 0 = NaN
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float fsqrt(float x) {
     float y;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 

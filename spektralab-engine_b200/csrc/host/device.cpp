@@ -28,8 +28,9 @@ struct DevBuffer::Impl {
     void* p = nullptr;
     size_t size = 0;
     std::shared_ptr<PoolState> pool;  // null: persistent (cudaMalloc)
+    bool borrowed = false;            // the caller's
     ~Impl() {
-        if (!p) return;
+        if (!p || borrowed) return;
         if (pool) {
             std::lock_guard<std::mutex> g(pool->m);
             cudaFreeAsync(p, pool->stream);
@@ -45,6 +46,15 @@ struct DevBuffer::Impl {
 
 void* DevBuffer::ptr() const { return p_ ? p_->p : nullptr; }
 size_t DevBuffer::size() const { return p_ ? p_->size : 0; }
+
+DevBuffer DevBuffer::borrow(void* p, size_t bytes) {
+    DevBuffer b;
+    b.p_ = std::make_shared<Impl>();
+    b.p_->p = p;
+    b.p_->size = bytes;
+    b.p_->borrowed = true;
+    return b;
+}
 
 Pool::Pool(cudaStream_t stream) : s_(std::make_shared<PoolState>()) { s_->stream = stream; }
 

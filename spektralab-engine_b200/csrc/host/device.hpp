@@ -34,6 +34,7 @@ public:
     size_t size() const;
     template <class T>
     T* as() const { return static_cast<T*>(ptr()); }
+    static DevBuffer borrow(void* p, size_t bytes);  // the caller's memory, which it frees after the last copy's use
 
 private:
     friend class Pool;

@@ -2029,8 +2029,11 @@ SPK_API spk_status spkx_print_negative(spk_session* session, const float* negati
         if (contraction && s.print_mode < 0)
             fail_invalid("the enlarger integral is written by the spectral-mode print kernel only");
         DeviceGuard dg(s.engine->device);
-        Plane neg = make_plane(s.pool, width, height);
-        cuda_check(cudaMemcpyAsync(neg.data(), negative, neg.bytes(), cudaMemcpyDeviceToDevice, s.stream), "negative");
+        // read where it lies: the print has read all of it before the scanner writes rgba16
+        Plane neg;
+        neg.buf = DevBuffer::borrow(const_cast<float*>(negative), size_t(width) * height * 3 * sizeof(float));
+        neg.w = width;
+        neg.h = height;
         OutputImage img{};
         img.dev = rgba16;
         img.width = width;
