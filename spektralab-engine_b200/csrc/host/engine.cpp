@@ -876,9 +876,9 @@ void launch_captured(Engine& e, const std::string& key, F&& body, cudaEvent_t t0
 
 // Enqueues the print side of the fused frames under `plan` on the batch stream (graph launch and, for the
 // persistent plans, the upload of the frame tables before it). Each fused frame's result is copied to its
-// pinned host image inside the graph, and frame_events[slot] marks its completion. In the per-frame plans
-// each frame waits inside the graph for its own negative (its ready event), so a frame prints while
-// later frames still develop; the persistent plans wait for every negative before their launch. The
+// pinned host image inside the graph, and frame_events[slot] marks its completion. A frame (per-frame
+// plans) or a group of frames (persistent plans) waits inside the graph for its own negatives (their ready
+// events), so it prints while later frames still develop. The
 // graph launch is bracketed by t0 and t1 when given.
 void run_plan(Engine& e, const std::string& plan, const std::string& shape, std::vector<BatchFrame>& fr,
               const std::vector<size_t>& slots, DevBuffer& tables, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = nullptr) {
@@ -909,7 +909,6 @@ void run_plan(Engine& e, const std::string& plan, const std::string& shape, std:
             t0, t1);
         return;
     }
-    for (size_t slot : slots) cuda_check(cudaStreamWaitEvent(bs, fr[slot].ready, 0), "frame ready");
     // persistent:S:C[:G]
     const size_t c1 = plan.find(':'), c2 = plan.find(':', c1 + 1), c3 = plan.find(':', c2 + 1);
     const uint32_t item_px = uint32_t(std::stoul(plan.substr(c1 + 1, c2 - c1 - 1)));
@@ -994,6 +993,9 @@ void run_plan(Engine& e, const std::string& plan, const std::string& shape, std:
             for (size_t g = 0; g < gl.size(); ++g) {
                 const GroupLayout& L = gl[g];
                 const BatchFrame& f0 = fr[slots[first[g]]];
+                // the group's own negatives: it prints, and its results go to the host, while later groups develop
+                for (size_t j = first[g]; j < first[g + 1]; ++j)
+                    cuda_check(cudaStreamWaitEvent(s, fr[slots[j]].ready, cudaEventWaitExternal), "frame ready");
                 dev::print_batch(reinterpret_cast<const BatchPrintFrame*>(d + L.o_pf),
                                  reinterpret_cast<const uint32_t*>(d + L.o_if),
                                  reinterpret_cast<const uint32_t*>(d + L.o_ip), L.n_items, item_px, ctas,
