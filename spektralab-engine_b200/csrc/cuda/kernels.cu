@@ -1105,10 +1105,13 @@ constexpr float kProductLockstep = 6.0f;
 // warp's ring as its slot alone, and the warp then takes 32 queued draws at a time, one attempt each, the
 // rejected queued again behind the rest; product-method draws (lambda < 10, or NaN) are set aside and run
 // last, so that a warp runs one method at a time. The kernel is bound by instruction issue (73 % of the
-// slots, 84 warp instructions a pixel): 4K benchmark frame 1.48 ms with ten-step bisections of the
-// densities' axis, general divides and the whole PTRS state in the ring, 0.83 this way.
-// Ten blocks per SM: 0.826 ms against 0.840 (nine), 0.865 (no cap); eleven slow the exports by 2 %.
-template <bool PACKED, bool PRODUCT>
+// slots, 83 warp instructions a pixel): 4K benchmark frame 1.48 ms with ten-step bisections of the
+// densities' axis, general divides and the whole PTRS state in the ring, 0.80 this way.
+// Ten blocks per SM: 0.826 ms against 0.840 (nine), 0.865 (no cap); eleven slow the exports by 2 %. Settling the
+// full test in the lockstep too (half as many queued draws) cost what it saved (0.84); a queue shared by
+// the block's warps lost more to its barriers (0.84 .. 0.90).
+// HOOK: the counts or lambdas are written out too (the adjoint, tests).
+template <bool PACKED, bool PRODUCT, bool HOOK>
 __global__ void __launch_bounds__(kDrawWarps * 32, SPKB_DEVELOP_MIN_BLOCKS) k_develop_layers(const float* __restrict__ exposure,
                                                                     float* __restrict__ out, uint32_t w,
                                                                     uint32_t blocks_per_row,
@@ -1120,7 +1123,7 @@ __global__ void __launch_bounds__(kDrawWarps * 32, SPKB_DEVELOP_MIN_BLOCKS) k_de
     const uint32_t x = (blockIdx.x - y * blocks_per_row) * (kDrawWarps * 32) + threadIdx.x;
     const bool live = x < w;
     const uint32_t pixel = y * q.width + x;
-    const size_t o = 3 * (size_t(y) * w + x);
+    const size_t o = 3 * (size_t(y) * w + min(x, w - 1));  // a lane past the row works on its last pixel, queues and stores nothing
     uint16_t* ringw = ring[wi];
     uint16_t* productw = product_list[wi];
     float* resw = lam[wi];
@@ -1129,17 +1132,15 @@ __global__ void __launch_bounds__(kDrawWarps * 32, SPKB_DEVELOP_MIN_BLOCKS) k_de
     uint32_t tail = 0;
 #pragma unroll
     for (uint32_t c = 0; c < 3; ++c) {
-        float dl[3] = {0.0f, 0.0f, 0.0f};
-        if (live) {
-            float L = log10f(fmaxf(exposure[o + c], 0.0f) + 1e-10f);
-            if (q.chi) L = __fsub_rn(L, q.chi[o + c]);  // DIR couplers: the corrected log exposure, the y0 curve
-            if (PACKED) {
-                const float D = curve_packed(q, c, L);
-                layers_packed(q, c, q.positive ? -D : D, dl);
-            } else {
-                const float D = curve_lookup(q.cx, q.cinv, q.cy + size_t(c) * q.K, q.K, q.cgrid, L);
-                layer_densities(q, c, q.positive ? -D : D, dl);
-            }
+        float dl[3];
+        float L = log10f(fmaxf(exposure[o + c], 0.0f) + 1e-10f);
+        if (q.chi) L = __fsub_rn(L, q.chi[o + c]);  // DIR couplers: the corrected log exposure, the y0 curve
+        if (PACKED) {
+            const float D = curve_packed(q, c, L);
+            layers_packed(q, c, q.positive ? -D : D, dl);
+        } else {
+            const float D = curve_lookup(q.cx, q.cinv, q.cy + size_t(c) * q.K, q.K, q.cgrid, L);
+            layer_densities(q, c, q.positive ? -D : D, dl);
         }
 #pragma unroll
         for (uint32_t l = 0; l < 3; ++l) {
@@ -1149,7 +1150,7 @@ __global__ void __launch_bounds__(kDrawWarps * 32, SPKB_DEVELOP_MIN_BLOCKS) k_de
             const float lm =
                 PACKED ? sublayer_lambda_fast(d, q.sat_d[lc], q.rcp_sat_d[lc], q.count[lc], q.uniformity[c], &sat)
                        : spk_sublayer_lambda(d, q.sat_d[lc], q.count[lc], q.uniformity[c], &sat);
-            if (q.lam_out && live) q.lam_out[size_t(pixel) * 9 + k] = lm;
+            if (HOOK && q.lam_out && live) q.lam_out[size_t(pixel) * 9 + k] = lm;
             scale[k][tid] = SPK_MUL(q.unit[lc], sat);  // unit: SPK_DIV(sat_d, count), formed once
             const spk_u4 words = philox_first(head0, q.stream_hi[k], q.stream_lo[k], q.seed);
             bool settled = squeeze_certain(lm, words.x, words.y, value);
@@ -1208,7 +1209,7 @@ __global__ void __launch_bounds__(kDrawWarps * 32, SPKB_DEVELOP_MIN_BLOCKS) k_de
 #pragma unroll
         for (int l = 0; l < 3; ++l) {
             const float cnt = resw[(c * 3 + l) * 32 + lane];
-            if (q.counts_out) q.counts_out[size_t(pixel) * 9 + c * 3 + l] = cnt;
+            if (HOOK && q.counts_out) q.counts_out[size_t(pixel) * 9 + c * 3 + l] = cnt;
             val[l] = SPK_MUL(cnt, scale[c * 3 + l][tid]);
         }
         float G = ((0.0f + val[0]) + val[1]) + val[2];
@@ -1499,9 +1500,14 @@ void develop(const float* exposure, float* out, const DevelopArgs& a, uint32_t w
         for (int i = 0; i < 9; ++i) mean += a.count[i] / 9.0f;
         const bool product = a.chi && mean < 160.0f;
         const dim3 g(bx * h), b(kDrawWarps * 32);
-        if (!a.packed) k_develop_layers<false, true><<<g, b, 0, s>>>(exposure, out, w, bx, a);
-        else if (product) k_develop_layers<true, true><<<g, b, 0, s>>>(exposure, out, w, bx, a);
-        else k_develop_layers<true, false><<<g, b, 0, s>>>(exposure, out, w, bx, a);
+        auto kernel = k_develop_layers<false, true, true>;
+        if (a.counts_out || a.lam_out) {
+            if (a.packed) kernel = product ? k_develop_layers<true, true, true> : k_develop_layers<true, false, true>;
+        } else {
+            kernel = k_develop_layers<false, true, false>;
+            if (a.packed) kernel = product ? k_develop_layers<true, true, false> : k_develop_layers<true, false, false>;
+        }
+        kernel<<<g, b, 0, s>>>(exposure, out, w, bx, a);
         return;
     }
     const dim3 b(32, 4), g(div_up(w, 32), div_up(h, 4));
