@@ -692,18 +692,22 @@ __global__ void __launch_bounds__(32) k_iir_v(float* work, float* out, const flo
 #pragma unroll 1
     for (uint32_t k = 0; k < nq; ++k) {
         if (k + 1 < nq) load(work, nxt, k + 1, false);
+        // the chain first, its results stored after it: a store would hold the next step back until the
+        // result's conversion is through
 #pragma unroll
         for (uint32_t j = 0; j < kColChunk; ++j) {
-            const uint32_t i = k * kColChunk + j;
-            if (i >= h) break;
             const double v = iir_step(kc, double(cur[j]), s1, s2, s3);
             s3 = s2;
             s2 = s1;
             s1 = v;
-            if (active) work[t + size_t(i) * stride] = float(v);
+            cur[j] = float(v);
         }
+        float* o = work + t + size_t(k * kColChunk) * stride;
 #pragma unroll
-        for (uint32_t j = 0; j < kColChunk; ++j) cur[j] = nxt[j];
+        for (uint32_t j = 0; j < kColChunk; ++j, o += stride) {
+            if (active && k * kColChunk + j < h) *o = cur[j];
+            cur[j] = nxt[j];
+        }
     }
     load(work, cur, 0, true);
     if (MODE == ACC_PLANE) load(acc, ca, 0, true);
@@ -718,20 +722,19 @@ __global__ void __launch_bounds__(32) k_iir_v(float* work, float* out, const flo
         }
 #pragma unroll
         for (uint32_t j = 0; j < kColChunk; ++j) {
-            const uint32_t i = k * kColChunk + j;
-            if (i >= h) break;
             const double v = iir_step(kc, double(cur[j]), s1, s2, s3);
             s3 = s2;
             s2 = s1;
             s1 = v;
-            const float y = float(v);
-            float r = y;
-            if (MODE == ACC_ZERO) r = 0.0f + wgt * y;
-            if (MODE == ACC_PLANE) r = ca[j] + wgt * y;
-            out[t + size_t(h - 1u - i) * stride] = active ? r : cur[j];
+            cur[j] = active ? float(v) : cur[j];
         }
 #pragma unroll
         for (uint32_t j = 0; j < kColChunk; ++j) {
+            const uint32_t i = k * kColChunk + j;
+            float r = cur[j];
+            if (MODE == ACC_ZERO && active) r = 0.0f + wgt * r;
+            if (MODE == ACC_PLANE && active) r = ca[j] + wgt * r;
+            if (i < h) out[t + size_t(h - 1u - i) * stride] = r;
             cur[j] = nxt[j];
             if (MODE == ACC_PLANE) ca[j] = na[j];
         }

@@ -495,11 +495,22 @@ Session* open_session(Engine& e, const void* data, bool device_ptr, uint32_t w, 
     // the frame: raw upload, then channels and non-finite values fixed on the device
     s->source = Plane{s->pool.acquire(size_t(npx) * 12), w, h};
     const size_t raw_bytes = size_t(npx) * ch * sizeof(float);
-    DevBuffer raw = s->pool.acquire(raw_bytes);
-    cuda_check(cudaMemcpyAsync(raw.ptr(), data, raw_bytes, device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                               s->stream),
-               "frame upload");
-    dev::source_copy(raw.as<float>(), s->source.data(), size_t(npx), ch, s->stream);
+    // a frame in this device's memory is read where it lies (the call waits for the pass below before it returns)
+    bool in_place = false;
+    if (device_ptr && reinterpret_cast<uintptr_t>(data) % sizeof(float) == 0) {
+        cudaPointerAttributes at{};
+        in_place = cudaPointerGetAttributes(&at, data) == cudaSuccess && at.type == cudaMemoryTypeDevice && at.device == e.device;
+        (void)cudaGetLastError();
+    }
+    DevBuffer raw;
+    if (!in_place) {
+        raw = s->pool.acquire(raw_bytes);
+        cuda_check(cudaMemcpyAsync(raw.ptr(), data, raw_bytes, device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                                   s->stream),
+                   "frame upload");
+    }
+    dev::source_copy(in_place ? static_cast<const float*>(data) : raw.as<float>(), s->source.data(), size_t(npx), ch,
+                     s->stream);
     cuda_check(cudaGetLastError(), "source copy");
 
     s->pipe = s->build(p, film, print);
