@@ -597,8 +597,10 @@ __device__ __forceinline__ void line_chunk(const float* src, float* dst, float* 
     }
 }
 
-__global__ void __launch_bounds__(32) k_iir_h(const float* __restrict__ in, float* out, uint32_t w, uint32_t h,
-                                              const __grid_constant__ IirCoefs q) {
+__global__ void __launch_bounds__(32) k_iir_h(uint32_t w, uint32_t h, const __grid_constant__ IirLineJobs jobs) {
+    const float* in = jobs.in[blockIdx.y];
+    float* out = jobs.work[blockIdx.y];
+    const IirCoefs& q = jobs.q[blockIdx.y];
     __shared__ float ring[kLineStages][kLineRows * kLinePitch];
     static_assert(3 * kLinePix == 96, "a row's chunk is three floats a lane");
     const uint32_t lane = threadIdx.x, r0 = blockIdx.x * kLineRows;
@@ -663,12 +665,15 @@ __global__ void __launch_bounds__(32) k_iir_h(const float* __restrict__ in, floa
 // Column pass of the line recurrence, a thread per line (neighbouring threads on neighbouring floats). Each
 // thread holds the next kColChunk samples in registers while it runs the current ones, so that a sample
 // costs its three dependent multiply-adds and no memory latency (6000 x 4000: 5.49 ms with a load per
-// sample, 0.66 this way). One-warp CTAs spread the lines over the SMs. A channel that is not filtered passes through.
+// sample, 0.65 this way). One-warp CTAs spread the lines over the SMs. A channel that is not filtered passes through.
 constexpr uint32_t kColChunk = 16;
 
 template <int MODE>
-__global__ void __launch_bounds__(32) k_iir_v(float* work, float* out, const float* acc, uint32_t w, uint32_t h,
-                                              const __grid_constant__ IirCoefs q, float w0, float w1, float w2) {
+__global__ void __launch_bounds__(32) k_iir_v(const float* acc, uint32_t w, uint32_t h,
+                                              const __grid_constant__ IirLineJobs jobs, float w0, float w1, float w2) {
+    float* work = jobs.work[blockIdx.y];
+    float* out = jobs.out[blockIdx.y];
+    const IirCoefs& q = jobs.q[blockIdx.y];
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 3u * w) return;
     const uint32_t c = t % 3u;
@@ -1448,18 +1453,43 @@ void fir_h(const float* in, float* out, const float* acc, uint32_t w, uint32_t h
     k_fir_h<<<g, b, 0, s>>>(in, out, acc, w, h, t, mode, weight[0], weight[1], weight[2]);
 }
 
-void iir_h(const float* in, float* out, uint32_t w, uint32_t h, const IirCoefs& c, cudaStream_t s) {
+void iir_h_lines(const IirLineJobs& j, uint32_t w, uint32_t h, cudaStream_t s) {
+    if (uint64_t(w) * h == 0 || j.n == 0) return;
     Probe p("iir_h", s);
-    k_iir_h<<<div_up(h, kLineRows), 32, 0, s>>>(in, out, w, h, c);
+    k_iir_h<<<dim3(div_up(h, kLineRows), j.n), 32, 0, s>>>(w, h, j);
+}
+
+void iir_v_lines(const IirLineJobs& j, uint32_t w, uint32_t h, cudaStream_t s) {
+    if (uint64_t(w) * h == 0 || j.n == 0) return;
+    Probe p("iir_v", s);
+    k_iir_v<ACC_NONE><<<dim3(div_up(3 * w, 32), j.n), 32, 0, s>>>(nullptr, w, h, j, 1.0f, 1.0f, 1.0f);
+}
+
+void iir_h(const float* in, float* out, uint32_t w, uint32_t h, const IirCoefs& c, cudaStream_t s) {
+    IirLineJobs j{};
+    j.n = 1;
+    j.in[0] = in;
+    j.work[0] = out;
+    j.q[0] = c;
+    iir_h_lines(j, w, h, s);
 }
 
 void iir_v(float* work, float* out, const float* acc, uint32_t w, uint32_t h, const IirCoefs& c, int mode,
            const float weight[3], cudaStream_t s) {
+    IirLineJobs j{};
+    j.n = 1;
+    j.work[0] = work;
+    j.out[0] = out;
+    j.q[0] = c;
+    if (mode == ACC_NONE) {
+        iir_v_lines(j, w, h, s);
+        return;
+    }
+    if (uint64_t(w) * h == 0) return;
     Probe p("iir_v", s);
     const uint32_t g = div_up(3 * w, 32);
-    if (mode == ACC_NONE) k_iir_v<ACC_NONE><<<g, 32, 0, s>>>(work, out, acc, w, h, c, weight[0], weight[1], weight[2]);
-    else if (mode == ACC_ZERO) k_iir_v<ACC_ZERO><<<g, 32, 0, s>>>(work, out, acc, w, h, c, weight[0], weight[1], weight[2]);
-    else k_iir_v<ACC_PLANE><<<g, 32, 0, s>>>(work, out, acc, w, h, c, weight[0], weight[1], weight[2]);
+    if (mode == ACC_ZERO) k_iir_v<ACC_ZERO><<<g, 32, 0, s>>>(acc, w, h, j, weight[0], weight[1], weight[2]);
+    else k_iir_v<ACC_PLANE><<<g, 32, 0, s>>>(acc, w, h, j, weight[0], weight[1], weight[2]);
 }
 
 void lincomb(const float* x, const float* y, float* out, size_t pixels, const float a[3], const float b[3],

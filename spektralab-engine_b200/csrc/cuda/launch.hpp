@@ -73,6 +73,10 @@ void iir_h(const float* in, float* out, uint32_t w, uint32_t h, const IirCoefs& 
 // pass; out := y, 0 + w y or acc + w y.
 void iir_v(float* work, float* out, const float* acc, uint32_t w, uint32_t h, const IirCoefs& c, int mode,
            const float weight[3], cudaStream_t s);
+// The row pass, or the column pass without accumulation, of j.n planes at once: a line pass of one plane keeps
+// only a warp or so per SM busy.
+void iir_h_lines(const IirLineJobs& j, uint32_t w, uint32_t h, cudaStream_t s);
+void iir_v_lines(const IirLineJobs& j, uint32_t w, uint32_t h, cudaStream_t s);
 // The recursive Gaussian of one direction with its tangent along sigma (the adjoint's sigma gradient):
 // (in, in_dot) -> (out, out_dot), dc the coefficients' derivatives; work planes hold the forward pass.
 void iir_tangent(const float* in, const float* in_dot, float* work, float* work_dot, float* out, float* out_dot,

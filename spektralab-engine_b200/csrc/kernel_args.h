@@ -46,6 +46,15 @@ struct IirCoefs {
     double B[3], B1[3], B2[3], B3[3];
 };
 
+// Line blurs of several planes of one size in one launch (iir_h_lines, iir_v_lines).
+struct IirLineJobs {
+    uint32_t n;
+    const float* in[SPKB_MAX_COMPONENTS];  // the row pass's input
+    float* work[SPKB_MAX_COMPONENTS];      // its result; the column pass overwrites it with its forward half
+    float* out[SPKB_MAX_COMPONENTS];       // the column pass's result
+    IirCoefs q[SPKB_MAX_COMPONENTS];
+};
+
 // Accumulation of a blur's last pass: out = v, out = 0 + w v, or out = acc + w v.
 enum AccMode { ACC_NONE = 0, ACC_ZERO = 1, ACC_PLANE = 2 };
 

@@ -58,3 +58,25 @@ def test_block_mixture_against_fp64(engine, lib, resources, w, h):
     f64 = setup_f64(lib, resources, delta, 35000.0 / max(w, h))["f64"]
     _, want = oracle.Oracle(f64, seed=1, halation=hal).render(img)
     np.testing.assert_allclose(neg, want, rtol=0, atol=5e-5)  # the float64 gate of the other negatives
+
+
+MIXED = {"run_first": [((0.4, 0.5, 0.6), (3.5, 2.0, 9.0)), ((0.2, 0.3, 0.4), (12.0, 14.0, 16.0)),
+                       ((0.5, 0.4, 0.3), (0.0, 5.0, 0.0))],
+         "run_after_fir": [((1.0, 0.8, 0.6), (0.6, 1.3, 2.9)), ((0.5, 0.4, 0.3), (0.0, 5.0, 1.1)),
+                           ((0.4, 0.5, 0.6), (3.5, 2.0, 9.0)), ((0.2, 0.3, 0.4), (0.7, 0.8, 0.9))],
+         "most": [((0.1, 0.2, 0.3), (3.0 + 0.5 * k, 0.4 * k, 4.0)) for k in range(8)]}
+
+
+@pytest.mark.parametrize("w,h", [(31, 33), (42, 64), (200, 97)])
+@pytest.mark.parametrize("name", sorted(MIXED))
+def test_joined_line_passes_against_fp64(engine, lib, resources, w, h, name):
+    """Components with recursive and FIR channels side by side: their line passes share launches."""
+    hal = (MIXED[name], (0.3, 0.2, 0.1))
+    delta = dict(BASE, grain_active=False)
+    img = sc.synthetic_image(w, h, 2)
+    with engine.open(img, delta) as s:
+        s.set_halation(*hal)
+        neg, _ = s.develop_debug("full", 1, w, h, counts=False)
+    f64 = setup_f64(lib, resources, delta, 35000.0 / max(w, h))["f64"]
+    _, want = oracle.Oracle(f64, seed=1, halation=hal).render(img)
+    np.testing.assert_allclose(neg, want, rtol=0, atol=5e-5)  # the float64 gate of the other negatives
