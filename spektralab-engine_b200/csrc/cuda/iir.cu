@@ -61,6 +61,16 @@ constexpr int kSegCols = SPKB_IIR_SEG_COLS;  // segments per column line (32: tw
 static_assert(kSegCols <= (1 << kIirScanSteps), "the carry scan composes at most 2^kIirScanSteps segments");
 constexpr int kColThreads = kColLines * kSegCols;
 
+// One pass's coefficients for up to N components, as a kernel argument: both passes of eight components by
+// value are 26 KB, which a small frame's launches copy longer than its blur takes.
+template <int N>
+struct IirPass {
+    int32_t seg_len, adjoint;
+    IirChannel ch[3 * N];
+    IirPass(const IirLaunch& q, uint32_t ncomp) : seg_len(q.seg_len), adjoint(q.adjoint) {
+        for (uint32_t i = 0; i < 3 * ncomp; ++i) ch[i] = q.ch[i];
+    }
+};
 
 // The column pass's tensor maps, one per component plane, and the strip's box geometry: `boxes` boxes of
 // `box_rows` rows (a multiple of 8, at most 256) cover the frame's rows; the strip buffer holds
@@ -223,7 +233,8 @@ __device__ __forceinline__ void edge_fold(const Coef& k, float* base, int e, int
 // handles line t / nseg, segment t % nseg when seg_major, else line t % nlines, segment t / nlines; the
 // channel of line j is 3 comp + j % 3. carry: shared scratch of 3 * nlines * nseg doubles, component i of
 // thread t's segment at carry[i * nlines * nseg + t].
-__device__ __forceinline__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, const IirLaunch& q, int comp,
+template <int N>
+__device__ __forceinline__ void blur_lines(float* buf, int pitch, int nlines, int n, int nseg, const IirPass<N>& q, int comp,
                            double* carry, bool seg_major) {
     const int t = threadIdx.x;
     const int line = seg_major ? t / nseg : t % nlines;
@@ -316,8 +327,10 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
+template <int N>
 __global__ void __launch_bounds__(kRowThreads) k_iir_rows(const float* __restrict__ in, const __grid_constant__ IirPlanes outs, uint32_t w,
-                                                          uint32_t h, const __grid_constant__ IirMixture mix) {
+                                                          uint32_t h, const __grid_constant__ IirSum mix,
+                                                          const __grid_constant__ IirPass<N> pass) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t y = blockIdx.x;
     if (y >= h) return;
@@ -338,7 +351,7 @@ __global__ void __launch_bounds__(kRowThreads) k_iir_rows(const float* __restric
         }
         cp_async_wait_all();
         __syncthreads();
-        blur_lines(work, 3, 3, int(w), kSegRows, mix.rows, c, carry, true);
+        blur_lines(work, 3, 3, int(w), kSegRows, pass, c, carry, true);
         float* dst = outs.p[c] + size_t(y) * p3;
         if ((p3 & 3) == 0) {
             for (int i = threadIdx.x; i < p3 / 4; i += blockDim.x)
@@ -411,7 +424,7 @@ __device__ __forceinline__ float mix2(float mx, float x, float my, float y) { re
 // tensor memory, or (to_strip) over the strip. Every lane of a warp with a quad left takes part in the
 // tensor-memory accesses; the quads past the frame's rows are the strip buffer's padding or its last row.
 template <bool MULTI>
-__device__ __forceinline__ void strip_sum(float* strip, int n, const IirMixture& mix, int c, uint32_t tmem, bool to_strip) {
+__device__ __forceinline__ void strip_sum(float* strip, int n, const IirSum& mix, int c, uint32_t tmem, bool to_strip) {
     const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads, last = n - 1;
     const QuadWeights wc = quad_weights(mix.weight[c]);
     uint32_t taddr = tmem + (uint32_t(32 * (warp & 3)) << 16) + 4u * uint32_t(warp >> 2);
@@ -430,7 +443,7 @@ __device__ __forceinline__ void strip_sum(float* strip, int n, const IirMixture&
 constexpr int kStoreBatch = 2;
 
 template <bool MULTI>
-__device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, size_t pitch, int n, const IirMixture& mix,
+__device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, size_t pitch, int n, const IirSum& mix,
                                              int c, uint32_t tmem) {
     const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads;
     const QuadWeights wc = quad_weights(mix.weight[c]), ma = quad_weights(mix.mix_a), mb = quad_weights(mix.mix_b);
@@ -469,7 +482,7 @@ __device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, siz
 // The same from a strip that holds the sum (or the plain blur) to a raw whose rows are not aligned, or a
 // strip cut by the frame's edge: a float at a time, nl to a row
 __device__ __forceinline__ void strip_to_raw_scalar(const float* strip, float* raw, size_t pitch, int nl, int n,
-                                                    const IirMixture& mix) {
+                                                    const IirSum& mix) {
     constexpr int kStep = kColThreads / kColLines, kBatch = 8;
     const int j = int(threadIdx.x) % kColLines;
     if (j >= nl) return;
@@ -494,9 +507,10 @@ __device__ __forceinline__ void strip_to_raw_scalar(const float* strip, float* r
 // MULTI: more than one component, the sum in tensor memory. Registers for two strips per SM (what shared
 // memory holds at 4K): held to three or four, even short frames ran slower (1024 x 1024, one component: 0.030 ms
 // at two, 0.035 and 0.038).
-template <bool MULTI>
+template <bool MULTI, int N>
 __global__ void __launch_bounds__(kColThreads, 2) k_iir_cols(float* raw, const __grid_constant__ IirPlanes hs, uint32_t w, uint32_t h,
-                                                          const __grid_constant__ IirMixture mix,
+                                                          const __grid_constant__ IirSum mix,
+                                                          const __grid_constant__ IirPass<N> pass,
                                                           const __grid_constant__ IirColMaps maps) {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t x0 = blockIdx.x * kColPixels;
@@ -570,7 +584,7 @@ __global__ void __launch_bounds__(kColThreads, 2) k_iir_cols(float* raw, const _
             }
         }
         __syncthreads();
-        blur_lines(strip, kColLines, kColLines, n, kSegCols, mix.cols, c, carry, false);
+        blur_lines(strip, kColLines, kColLines, n, kSegCols, pass, c, carry, false);
         if (MULTI && c + 1 < int(mix.ncomp)) {
             strip_sum<MULTI>(strip, n, mix, c, tmem, false);
         } else if (raw_vec) {
@@ -706,6 +720,24 @@ bool col_maps(IirColMaps& maps, const IirPlanes& planes, uint32_t ncomp, uint32_
     maps.use_tma = 1;
     return true;
 }
+
+template <int N>
+void launch_passes(const float* src, float* raw, const IirPlanes& planes, uint32_t w, uint32_t h, const IirMixture& m,
+                   const IirColMaps& maps, cudaStream_t s) {
+    const size_t sr = iir_rows_smem(m.pitch), sc = iir_cols_smem(h);
+    constexpr bool kMulti = N > 1;
+    ensure_smem(reinterpret_cast<const void*>(k_iir_rows<N>), int(sr));
+    ensure_smem(reinterpret_cast<const void*>(k_iir_cols<kMulti, N>), int(sc));
+    {
+        Probe p("iir_rows", s);
+        k_iir_rows<N><<<h, kRowThreads, sr, s>>>(src, planes, w, h, m, IirPass<N>(m.rows, m.ncomp));
+    }
+    {
+        Probe p("iir_cols", s);
+        const uint32_t g = (w + kColPixels - 1) / kColPixels;
+        k_iir_cols<kMulti, N><<<g, kColThreads, sc, s>>>(raw, planes, w, h, m, IirPass<N>(m.cols, m.ncomp), maps);
+    }
+}
 }  // namespace
 
 void set_iir_wait_limit(long long cycles) { g_wait_limit.store(cycles); }
@@ -722,29 +754,17 @@ void iir_mixture(const float* src, float* raw, float* const* tmp, uint32_t w, ui
                  cudaStream_t s) {
     IirPlanes planes{};
     for (uint32_t c = 0; c < m.ncomp; ++c) planes.p[c] = tmp[c];
-    const size_t sr = iir_rows_smem(m.pitch), sc = iir_cols_smem(h);
-    ensure_smem(reinterpret_cast<const void*>(k_iir_rows), int(sr));
-    const bool multi = m.ncomp > 1;
-    ensure_smem(multi ? reinterpret_cast<const void*>(k_iir_cols<true>) : reinterpret_cast<const void*>(k_iir_cols<false>),
-                int(sc));
     IirColMaps maps{};
     col_maps(maps, planes, m.ncomp, m.pitch, h);
-    if (multi) {
+    if (m.ncomp > 1) {
         // four columns for every 128 quads; allocations are powers of two from 32
         const uint32_t need = 4u * ((3u * h + 127u) / 128u);
         maps.tmem_cols = 32;
         while (maps.tmem_cols < need) maps.tmem_cols *= 2;
     }
-    {
-        Probe p("iir_rows", s);
-        k_iir_rows<<<h, kRowThreads, sr, s>>>(src, planes, w, h, m);
-    }
-    {
-        Probe p("iir_cols", s);
-        const uint32_t g = (w + kColPixels - 1) / kColPixels;
-        if (multi) k_iir_cols<true><<<g, kColThreads, sc, s>>>(raw, planes, w, h, m, maps);
-        else k_iir_cols<false><<<g, kColThreads, sc, s>>>(raw, planes, w, h, m, maps);
-    }
+    if (m.ncomp == 1) launch_passes<1>(src, raw, planes, w, h, m, maps, s);
+    else if (m.ncomp == 2) launch_passes<2>(src, raw, planes, w, h, m, maps, s);
+    else launch_passes<SPKB_MAX_COMPONENTS>(src, raw, planes, w, h, m, maps, s);
 }
 
 }  // namespace spkb::dev

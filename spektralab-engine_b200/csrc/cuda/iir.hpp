@@ -29,7 +29,8 @@ struct IirLaunch {
     IirChannel ch[3 * SPKB_MAX_COMPONENTS];  // [component * 3 + channel]
 };
 
-struct IirMixture {
+// What both passes need beside the coefficients
+struct IirSum {
     uint32_t ncomp;
     // 1: a plain blur, raw := G_0(src) with one component (weight, mix_a and mix_b unused); the column
     // pass stores the blurred lines as they are and never reads raw
@@ -37,6 +38,9 @@ struct IirMixture {
     float weight[SPKB_MAX_COMPONENTS][3];
     uint32_t pitch;  // pixels per row of the tmp planes, at least the frame's width (iir_pitch)
     float mix_a[3], mix_b[3];  // raw := mix_a raw + mix_b sum_k weight_k G_k(raw)
+};
+
+struct IirMixture : IirSum {
     IirLaunch rows, cols;
 };
 
