@@ -1,5 +1,7 @@
 #include "device.hpp"
 
+#include <cuda.h>
+
 #include <atomic>
 #include <cstdint>
 #include <vector>
@@ -117,6 +119,27 @@ DevBuffer Pool::persistent(size_t bytes) {
 size_t Pool::live_bytes() const {
     std::lock_guard<std::mutex> g(s_->m);
     return s_->live;
+}
+
+bool readable_in_place(const void* p, size_t bytes, int device) {
+    using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const Range range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Range>(f);
+    }();
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    cudaPointerAttributes a{};
+    const bool here = range && at % 16 == 0 && cudaPointerGetAttributes(&a, p) == cudaSuccess &&
+                      a.type == cudaMemoryTypeDevice && a.device == device;
+    (void)cudaGetLastError();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    return here && range(&base, &size, CUdeviceptr(at)) == CUDA_SUCCESS && at >= base && bytes <= size &&
+           at - base <= size - bytes;
 }
 
 void configure_device_pool(int device) {

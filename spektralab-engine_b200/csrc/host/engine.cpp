@@ -496,12 +496,7 @@ Session* open_session(Engine& e, const void* data, bool device_ptr, uint32_t w, 
     s->source = Plane{s->pool.acquire(size_t(npx) * 12), w, h};
     const size_t raw_bytes = size_t(npx) * ch * sizeof(float);
     // a frame in this device's memory is read where it lies (the call waits for the pass below before it returns)
-    bool in_place = false;
-    if (device_ptr && reinterpret_cast<uintptr_t>(data) % sizeof(float) == 0) {
-        cudaPointerAttributes at{};
-        in_place = cudaPointerGetAttributes(&at, data) == cudaSuccess && at.type == cudaMemoryTypeDevice && at.device == e.device;
-        (void)cudaGetLastError();
-    }
+    const bool in_place = device_ptr && readable_in_place(data, raw_bytes, e.device);
     DevBuffer raw;
     if (!in_place) {
         raw = s->pool.acquire(raw_bytes);
@@ -2042,9 +2037,16 @@ SPK_API spk_status spkx_print_negative(spk_session* session, const float* negati
         if (contraction && s.print_mode < 0)
             fail_invalid("the enlarger integral is written by the spectral-mode print kernel only");
         DeviceGuard dg(s.engine->device);
-        // read where it lies: the print has read all of it before the scanner writes rgba16
+        // read where it lies if it can be: the print has read all of it before the scanner writes rgba16 (the
+        // integral is written while the print reads, so with it the negative is copied: the two may overlap)
+        const size_t bytes = size_t(width) * height * 3 * sizeof(float);
         Plane neg;
-        neg.buf = DevBuffer::borrow(const_cast<float*>(negative), size_t(width) * height * 3 * sizeof(float));
+        if (!contraction && readable_in_place(negative, bytes, s.engine->device)) {
+            neg.buf = DevBuffer::borrow(const_cast<float*>(negative), bytes);
+        } else {
+            neg.buf = s.pool.acquire(bytes);
+            cuda_check(cudaMemcpyAsync(neg.buf.ptr(), negative, bytes, cudaMemcpyDeviceToDevice, s.stream), "negative");
+        }
         neg.w = width;
         neg.h = height;
         OutputImage img{};
