@@ -1113,8 +1113,8 @@ __global__ void __launch_bounds__(kDrawWarps * 32, SPKB_DEVELOP_MIN_BLOCKS) k_de
     __shared__ uint16_t ring[kDrawWarps][kDrawRing], product_list[kDrawWarps][9 * 32];
     __shared__ float lam[kDrawWarps][9 * 32], scale[9][kDrawWarps * 32];  // [c * 3 + l]; a count replaces its lambda
     const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5, tid = threadIdx.x;
-    const uint32_t y = blockIdx.x / blocks_per_row;
-    const uint32_t x = (blockIdx.x - y * blocks_per_row) * (kDrawWarps * 32) + threadIdx.x;
+    const uint32_t row = blockIdx.x / blocks_per_row, y = q.row0 + row;
+    const uint32_t x = (blockIdx.x - row * blocks_per_row) * (kDrawWarps * 32) + threadIdx.x;
     const bool live = x < w;
     const uint32_t pixel = y * q.width + x;
     const size_t o = 3 * (size_t(y) * w + min(x, w - 1));  // a lane past the row works on its last pixel, queues and stores nothing
@@ -1531,6 +1531,13 @@ void develop(const float* exposure, float* out, const DevelopArgs& a, uint32_t w
     const dim3 b(32, 4), g(div_up(w, 32), div_up(h, 4));
     Probe p("develop", s);
     k_develop<<<g, b, 0, s>>>(exposure, out, w, h, a);
+}
+
+void develop_rows(const float* exposure, float* out, const DevelopArgs& a, uint32_t w, uint32_t row0, uint32_t rows,
+                  cudaStream_t s) {
+    DevelopArgs b = a;
+    b.row0 = row0;
+    develop(exposure, out, b, w, rows, s);
 }
 
 void coupler_source(const float* exposure, float* chi, const CouplerArgs& a, cudaStream_t s) {

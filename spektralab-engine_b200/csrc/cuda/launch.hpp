@@ -91,6 +91,9 @@ void coupler_source(const float* exposure, float* chi, const CouplerArgs& a, cud
 
 // log10 exposure -> density curves -> grain draw (grain mode) or density (no grain).
 void develop(const float* exposure, float* out, const DevelopArgs& a, uint32_t w, uint32_t h, cudaStream_t s);
+// Rows row0 .. row0 + rows - 1 of the same frame's sub-layer grain (a.grain, mode 0): the draws are per pixel
+void develop_rows(const float* exposure, float* out, const DevelopArgs& a, uint32_t w, uint32_t row0, uint32_t rows,
+                  cudaStream_t s);
 // The grain's log(k!) table on the current device (once per process; waits for it on s). The engine calls
 // it at creation; develop calls it too, before its first grain launch on a device.
 void develop_prepare(cudaStream_t s);
@@ -132,6 +135,10 @@ constexpr uint32_t scan_tile_rows() { return 32; }
 // out must not alias in. fir_tile_fits tells whether the tiled kernel takes this frame and radius.
 bool fir_tile_fits(uint32_t w, uint32_t h, int r);
 void fir_tile(const float* in, float* out, uint32_t w, uint32_t h, int r, const float* taps, cudaStream_t s);
+// Rows row0 .. row1 - 1 of it, row0 a multiple of kFirTileRows; in is read up to r rows past them
+constexpr uint32_t kFirTileRows = 32;
+void fir_tile_rows(const float* in, float* out, uint32_t w, uint32_t h, uint32_t row0, uint32_t row1, int r,
+                   const float* taps, cudaStream_t s);
 
 // A run of a.n separable FIRs of one plane with per-channel taps, every pass of all of them in one tiled
 // kernel: out := G(in) (one component, ACC_NONE), or out := (0 or acc) + sum_k weight_k G_k(in), the terms

@@ -253,13 +253,13 @@ __global__ void __launch_bounds__(kThreads) k_scan_encode_batch(const BatchScanF
 // pass. out must not alias in (neighbouring tiles read in's halo).
 template <int R>
 __global__ void __launch_bounds__(kThreads) k_fir_tile(const float* __restrict__ in, float* __restrict__ out, int w,
-                                                       int h, const __grid_constant__ ScanArgs a) {
+                                                       int h, int row0, const __grid_constant__ ScanArgs a) {
     extern __shared__ float smem[];
     const int r = R >= 0 ? R : a.r1;
     const int PC = 3 * (kTW + 2 * r), PR = kTH + 2 * r;
     float* A = smem;
     float* B = smem + PR * PC;
-    const int x0 = blockIdx.x * kTW, y0 = blockIdx.y * kTH;
+    const int x0 = blockIdx.x * kTW, y0 = row0 + int(blockIdx.y) * kTH;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool inner_x = x0 - r >= 0 && x0 + kTW + r <= w;  // the haloed columns lie inside the frame
     for (int i = warp; i < PR; i += kWarps) {
@@ -538,25 +538,32 @@ void scan_encode_batch(const BatchScanFrame* frames, uint32_t n_frames, uint32_t
 
 namespace {
 template <int R>
-void launch_fir_tile(const float* in, float* out, uint32_t w, uint32_t h, const ScanArgs& a, cudaStream_t s) {
+void launch_fir_tile(const float* in, float* out, uint32_t w, uint32_t h, uint32_t row0, uint32_t row1, const ScanArgs& a,
+                     cudaStream_t s) {
     const size_t smem = size_t(2 * kTH + 2 * a.r1) * size_t(3 * (kTW + 2 * a.r1)) * sizeof(float);
     ensure_smem(reinterpret_cast<const void*>(k_fir_tile<R>), int(smem));
-    const dim3 g((w + kTW - 1) / kTW, (h + kTH - 1) / kTH);
-    k_fir_tile<R><<<g, kThreads, smem, s>>>(in, out, int(w), int(h), a);
+    const dim3 g((w + kTW - 1) / kTW, (row1 - row0 + kTH - 1) / kTH);
+    k_fir_tile<R><<<g, kThreads, smem, s>>>(in, out, int(w), int(h), int(row0), a);
 }
 }  // namespace
 
 bool fir_tile_fits(uint32_t w, uint32_t h, int r) { return scan_encode_fits(w, h, r, 0); }
 
 void fir_tile(const float* in, float* out, uint32_t w, uint32_t h, int r, const float* taps, cudaStream_t s) {
-    if (uint64_t(w) * h == 0) return;
+    fir_tile_rows(in, out, w, h, 0, h, r, taps, s);
+}
+
+void fir_tile_rows(const float* in, float* out, uint32_t w, uint32_t h, uint32_t row0, uint32_t row1, int r,
+                   const float* taps, cudaStream_t s) {
+    static_assert(kFirTileRows == uint32_t(kTH), "a row range starts at a tile");
+    if (uint64_t(w) * (row1 - row0) == 0) return;
     ScanArgs a{};
     a.r1 = r;
     for (int k = 0; k <= 2 * r; ++k) a.t1[k] = taps[k];
     Probe p("fir_tile", s);
-    if (r == 2) launch_fir_tile<2>(in, out, w, h, a, s);
-    else if (r == 5) launch_fir_tile<5>(in, out, w, h, a, s);
-    else launch_fir_tile<-1>(in, out, w, h, a, s);
+    if (r == 2) launch_fir_tile<2>(in, out, w, h, row0, row1, a, s);
+    else if (r == 5) launch_fir_tile<5>(in, out, w, h, row0, row1, a, s);
+    else launch_fir_tile<-1>(in, out, w, h, row0, row1, a, s);
 }
 
 void fir_mixture(const float* in, float* out, const float* acc, uint32_t w, uint32_t h, const FirMixArgs& a,

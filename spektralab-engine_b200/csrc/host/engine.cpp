@@ -572,6 +572,7 @@ void render(Session& s, const char* tier_name, bool reprint, spk_result* out) {
         ctx.print_bins = s.print_bins;
         if (!reuse) {
             developed = true;
+            ctx.defer_grain = true;
             develop_tier(s, *t, ctx);
         }
         ctx.print_seed = s.draw_print_seed();

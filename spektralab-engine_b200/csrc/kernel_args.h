@@ -109,6 +109,7 @@ struct DevelopArgs {
     float curve_last, axis_last[3];  // the axes' last points
     float guide_x0[3], guide_s[3];
     uint32_t width;       // pixel index = y * width + x keys the draws
+    uint32_t row0;        // the launch's first row (develop_rows; 0 otherwise)
     float* counts_out;    // test hook: the Poisson counts, [pixel][c][l]; nullptr in renders
     float* lam_out;       // test hook: the draws' lambdas, [pixel][c][l] (sub-layer grain); nullptr in renders
     // DIR couplers: the blurred correction plane chi (interleaved RGB), subtracted from the log exposure
