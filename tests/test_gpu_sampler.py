@@ -1,0 +1,25 @@
+"""The grain sampler on the device against its host build, bit for bit, where its branch-free operations
+would leave their range: lambdas at the ends of binary32."""
+
+import numpy as np
+import pytest
+
+import oracle
+from conftest import sc
+
+pytestmark = pytest.mark.gpu
+
+
+def device_poisson(lib, lam, stream, seed):
+    lam = np.ascontiguousarray(lam, np.float32)
+    out = np.zeros_like(lam)
+    lib.check(lib.lib.spkx_sampler_poisson(lam.ctypes.data_as(sc.FP), out.ctypes.data_as(sc.FP), lam.size, stream, seed))
+    return out
+
+
+@pytest.mark.parametrize("lam", [np.inf, -np.inf, np.nan, np.finfo(np.float32).max, 1e30, 1e20, 0.0, -3.0, 1e-45, 10.0,
+                                 np.nextafter(np.float32(10), np.float32(0))])
+def test_lambda_at_the_ends_of_binary32(lib, lam):
+    lam = np.full(4099, lam, np.float32)
+    for stream, seed in ((0, 1), (21, 77)):
+        np.testing.assert_array_equal(device_poisson(lib, lam, stream, seed), oracle.poisson(lam, stream, seed))
