@@ -94,6 +94,12 @@ SPK_API spk_status spkx_setup_json(const char* resources_dir, const char* params
 /* Poisson counts (as floats) of the grain sampler for pixel index i = 0..n-1 on one stream and seed */
 SPK_API spk_status spkx_sampler_poisson(const float* lam, float* counts, uint32_t n, uint32_t stream,
                                         uint32_t seed);
+/* the sampler's branch-free operations against the compiler's correctly rounded ones: *wrong receives how many of n
+ * results differ. op 0: the reciprocal, item i with significand i mod 2^23 and exponent (i >> 23) - 100, n at
+ * most 201 2^23; 1: the square root, the same items, n at most 227 2^23; 2: the quotient and 3: the quotient by
+ * a constant's reciprocal, of random operands, every other result next to the middle of two floats, n at most
+ * 2^32. SPK_ERR_INVALID_ARG for another op or a larger n. */
+SPK_API spk_status spkx_test_sampler_ops(int32_t op, uint64_t n, uint32_t seed, uint64_t* wrong);
 /* the Box-Muller lognormal value for pixel index i = 0..n-1 */
 SPK_API spk_status spkx_sampler_lognormal(float* out, uint32_t n, float mean, float stddev, uint32_t stream,
                                           uint32_t seed);

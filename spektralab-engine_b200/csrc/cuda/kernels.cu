@@ -10,6 +10,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -1078,12 +1079,18 @@ __device__ __forceinline__ void layers_packed(const DevelopArgs& q, uint32_t c, 
     for (int l = 0; l < 3; ++l) dl[l] = t[2 + 2 * l] + f * t[3 + 2 * l];
 }
 
-// spk_sublayer_lambda with the quotients by a constant's reciprocal (exact after its remainder's
-// correction: Brisebarre, Muller and Raina, "Accelerating correctly rounded floating-point division when
-// the divisor is known in advance", IEEE Trans. Computers 53 (2004)) and by spk_div_normal
-__device__ __forceinline__ float sublayer_lambda_fast(float d, float D, float rD, float n, float u, float* sat_out) {
+// d / D correctly rounded from D's correctly rounded reciprocal rD, exact after the remainder's correction:
+// Brisebarre, Muller and Raina, "Accelerating correctly rounded floating-point division when the divisor is
+// known in advance", IEEE Trans. Computers 53 (2004). For quotients and remainders clear of underflow.
+__device__ __forceinline__ float div_by_constant(float d, float D, float rD) {
     const float q0 = __fmul_rn(d, rD);
-    float q = __fmaf_rn(__fmaf_rn(-q0, D, d), rD, q0);
+    return __fmaf_rn(__fmaf_rn(-q0, D, d), rD, q0);
+}
+
+// spk_sublayer_lambda with the quotients by div_by_constant (one small enough to underflow is clamped to
+// 1e-6 in any case) and by spk_div_normal
+__device__ __forceinline__ float sublayer_lambda_fast(float d, float D, float rD, float n, float u, float* sat_out) {
+    float q = div_by_constant(d, D, rD);
     q = q < 1e-6f ? 1e-6f : (q > 0.999999f ? 0.999999f : q);
     const float sat = SPK_SUB(1.0f, SPK_MUL(SPK_MUL(q, u), 0.999999f));
     *sat_out = sat;
@@ -1269,6 +1276,43 @@ __global__ void k_sampler_poisson(const float* lam, float* out, uint32_t n, uint
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     out[i] = spk_poisson(lam[i], i, stream, seed);
+}
+
+// The sampler's branch-free operations against the compiler's correctly rounded ones: how many of n results
+// differ (SamplerOp).
+__device__ __forceinline__ float ldexp_bits(uint32_t significand, int e) {
+    return __uint_as_float(uint32_t(127 + e) << 23 | (significand & 0x007FFFFFu));
+}
+
+__global__ void k_sampler_ops(int op, uint64_t n, uint32_t seed, unsigned long long* wrong) {
+    uint32_t bad = 0;
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
+        if (op == SAMPLER_OP_RCP || op == SAMPLER_OP_SQRT) {  // every significand, exponents from -100 up
+            const float x = ldexp_bits(uint32_t(i), int(i >> 23) - 100);
+            const float got = op == SAMPLER_OP_RCP ? SPK_RCP_NORMAL(x) : SPK_SQRT_NORMAL(x);
+            const float want = op == SAMPLER_OP_RCP ? __frcp_rn(x) : __fsqrt_rn(x);
+            bad += __float_as_uint(got) != __float_as_uint(want);
+            continue;
+        }
+        spk_u4 c;
+        c.x = uint32_t(i);
+        c.y = uint32_t(i >> 32);
+        c.z = uint32_t(op);
+        c.w = 0u;
+        const spk_u4 r = spk_philox(c, seed, 0u);
+        float a = ldexp_bits(r.x, int(r.z % 81u) - 40), b = ldexp_bits(r.y, int(r.w % 121u) - 60);
+        if (i & 1u) {
+            // a quotient as near the middle of two floats as a 24-bit numerator allows: a = b times an odd
+            // 25-bit number, cut to 24 bits, or the next float above
+            const uint64_t Q = 0x1000001u | (r.x & 0xFFFFFFu), P = Q * (0x800000u | (r.y & 0x7FFFFFu));
+            const uint32_t A = uint32_t(P >> (40 - __clzll((long long)P))) + uint32_t((i >> 1) & 1u);
+            a = float(A);
+        }
+        const float want = __fdiv_rn(a, b);
+        const float got = op == SAMPLER_OP_DIV ? SPK_DIV_NORMAL(a, b) : div_by_constant(a, b, __frcp_rn(b));
+        bad += __float_as_uint(got) != __float_as_uint(want);
+    }
+    if (bad) atomicAdd(wrong, (unsigned long long)bad);
 }
 
 // The print glare's field (reference kernels/fx_grain.metal:99-116 with same_all): one lognormal value
@@ -1568,6 +1612,12 @@ void sampler_poisson(const float* lam, float* out, uint32_t n, uint32_t stream, 
     if (n == 0) return;
     Probe p("sampler_poisson", s);
     k_sampler_poisson<<<div_up(n, 128), 128, 0, s>>>(lam, out, n, stream, seed);
+}
+
+void sampler_ops(int op, uint64_t n, uint32_t seed, unsigned long long* wrong, cudaStream_t s) {
+    if (n == 0) return;
+    Probe p("sampler_ops", s);
+    k_sampler_ops<<<unsigned(std::min<uint64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(op, n, seed, wrong);
 }
 
 void glare_field(float* out, uint32_t pixels, float mean, float sd, uint32_t seed, cudaStream_t s) {

@@ -169,6 +169,14 @@ void fill(void* p, size_t bytes, uint32_t v, cudaStream_t s);
 
 // Test entry points: the sampler over an array of lambdas (counts as floats) and raw Philox blocks.
 void sampler_poisson(const float* lam, float* out, uint32_t n, uint32_t stream, uint32_t seed, cudaStream_t s);
+// The sampler's branch-free operations: adds to *wrong how many of n results differ from the compiler's
+enum SamplerOp {
+    SAMPLER_OP_RCP = 0,   // item i: significand i mod 2^23, exponent (i >> 23) - 100
+    SAMPLER_OP_SQRT = 1,  // the same
+    SAMPLER_OP_DIV = 2,   // random operands, every other quotient next to the middle of two floats
+    SAMPLER_OP_DIV_CONST = 3,
+};
+void sampler_ops(int op, uint64_t n, uint32_t seed, unsigned long long* wrong, cudaStream_t s);
 void sampler_lognormal(float* out, uint32_t n, float mean, float stddev, uint32_t stream, uint32_t seed,
                        cudaStream_t s);
 void philox_blocks(const uint32_t* ctr, const uint32_t* key, uint32_t* out, uint32_t n, cudaStream_t s);

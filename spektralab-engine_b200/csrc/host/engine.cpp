@@ -2577,6 +2577,23 @@ SPK_API spk_status spkx_sampler_poisson(const float* lam, float* counts, uint32_
     });
 }
 
+SPK_API spk_status spkx_test_sampler_ops(int32_t op, uint64_t n, uint32_t seed, uint64_t* wrong) {
+    last_error::clear();
+    if (!wrong) return invalid("wrong is NULL");
+    // exponents up to 2^100 for the reciprocal's, to the largest for the root's
+    const uint64_t most[] = {uint64_t(201) << 23, uint64_t(227) << 23, uint64_t(1) << 32, uint64_t(1) << 32};
+    if (op < 0 || op > 3 || n > most[op]) return invalid("no such operation, or more items than its range has");
+    return with_scratch_stream([&](cudaStream_t s) {
+        DevArray d(sizeof(unsigned long long));
+        unsigned long long w = 0;
+        cuda_check(cudaMemsetAsync(d.p, 0, sizeof w, s), "memset");
+        dev::sampler_ops(op, n, seed, static_cast<unsigned long long*>(d.p), s);
+        cuda_check(cudaMemcpyAsync(&w, d.p, sizeof w, cudaMemcpyDeviceToHost, s), "copy");
+        cuda_check(cudaStreamSynchronize(s), "sampler operations");
+        *wrong = w;
+    });
+}
+
 SPK_API spk_status spkx_sampler_lognormal(float* out, uint32_t n, float mean, float stddev, uint32_t stream,
                                           uint32_t seed) {
     last_error::clear();

@@ -97,6 +97,7 @@ EXT = {
     "spkx_session_tier_image": (I32, [P, C, FP, ctypes.c_size_t, ctypes.POINTER(U32), ctypes.POINTER(U32)]),
     "spkx_session_setup_json": (I32, [P, ctypes.c_double, PS]),
     "spkx_sampler_poisson": (I32, [FP, FP, U32, U32, U32]),
+    "spkx_test_sampler_ops": (I32, [I32, ctypes.c_uint64, U32, ctypes.POINTER(ctypes.c_uint64)]),
     "spkx_sampler_lognormal": (I32, [FP, U32, ctypes.c_float, ctypes.c_float, U32, U32]),
     "spkx_philox": (I32, [UP, UP, UP, U32]),
     "spkx_gaussian": (I32, [FP, FP, U32, U32, DP]),

@@ -1,5 +1,7 @@
 """The grain sampler on the device against its host build, bit for bit, where its branch-free operations
-would leave their range: lambdas at the ends of binary32."""
+would leave their range: lambdas at the ends of binary32. And those operations against the compiler's."""
+
+import ctypes
 
 import numpy as np
 import pytest
@@ -23,3 +25,16 @@ def test_lambda_at_the_ends_of_binary32(lib, lam):
     lam = np.full(4099, lam, np.float32)
     for stream, seed in ((0, 1), (21, 77)):
         np.testing.assert_array_equal(device_poisson(lib, lam, stream, seed), oracle.poisson(lam, stream, seed))
+
+
+RCP, SQRT, DIV, DIV_CONST = range(4)
+
+
+@pytest.mark.parametrize("op,n,seed", [(RCP, 201 << 23, 0), (SQRT, 227 << 23, 0), (DIV, 1 << 31, 1), (DIV, 1 << 31, 2),
+                                       (DIV_CONST, 1 << 31, 3)])
+def test_operations_correctly_rounded(lib, op, n, seed):
+    """The reciprocal and the root over every significand and exponent that they are used at; the quotients,
+    which have two significands, over random ones and those nearest a rounding boundary."""
+    wrong = ctypes.c_uint64(1)
+    lib.check(lib.lib.spkx_test_sampler_ops(op, n, seed, ctypes.byref(wrong)))
+    assert wrong.value == 0
