@@ -1,5 +1,5 @@
 """The grain sampler on the device against its host build, bit for bit, where its branch-free operations
-would leave their range: lambdas at the ends of binary32. And those operations against the compiler's."""
+would leave their range: lambdas at the ends of binary32, a uniform of 1. And those operations against the compiler's."""
 
 import ctypes
 
@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle
-from conftest import sc
+from conftest import BASE, sc
 
 pytestmark = pytest.mark.gpu
 
@@ -25,6 +25,24 @@ def test_lambda_at_the_ends_of_binary32(lib, lam):
     lam = np.full(4099, lam, np.float32)
     for stream, seed in ((0, 1), (21, 77)):
         np.testing.assert_array_equal(device_poisson(lib, lam, stream, seed), oracle.poisson(lam, stream, seed))
+
+
+# (seed, c, l, pixel) whose draw (c, l) starts with a word of 24 leading ones: the squeeze divides by us = 0
+TOP_WORDS = [(332, 1, 0, 561), (1155, 2, 1, 1383), (2857, 0, 0, 1755), (3815, 2, 2, 1706)]
+
+
+@pytest.mark.parametrize("seed,c,l,pixel", TOP_WORDS)
+def test_uniform_of_one(lib, engine, seed, c, l, pixel):
+    """The attempt is rejected by the sampler and by the develop kernel's queue, whatever its candidate was."""
+    assert int(sc.philox_np([pixel], [c + 10 * l], seed)[0]) >> 8 == 0xFFFFFF
+    for lam in (10.0, 37.0, 2500.0, 1e5):
+        lam = np.full(pixel + 1, lam, np.float32)
+        np.testing.assert_array_equal(device_poisson(lib, lam, c + 10 * l, seed), oracle.poisson(lam, c + 10 * l, seed))
+    with engine.open(sc.synthetic_image(64, 64, 6), dict(BASE, film_format_mm=4.0)) as s:
+        counts, lam = s.develop_draws("full", seed, 64, 64)
+    want = oracle.poisson(lam[..., 3 * c + l].ravel(), c + 10 * l, seed)
+    assert lam[..., 3 * c + l].ravel()[pixel] >= 10.0
+    np.testing.assert_array_equal(counts[..., 3 * c + l].ravel(), want)
 
 
 RCP, SQRT, DIV, DIV_CONST = range(4)
