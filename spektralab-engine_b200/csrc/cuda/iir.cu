@@ -422,7 +422,8 @@ __device__ __forceinline__ float mix2(float mx, float x, float my, float y) { re
 
 // The blurred strip of component c joins the sum: acc := 0 + w v or acc + w v. The result goes back to the
 // tensor memory, or (to_strip) over the strip. Every lane of a warp with a quad left takes part in the
-// tensor-memory accesses; the quads past the frame's rows are the strip buffer's padding or its last row.
+// tensor-memory accesses, those past the frame's rows with zeros: a strip row is read and written by its
+// owner alone.
 template <bool MULTI>
 __device__ __forceinline__ void strip_sum(float* strip, int n, const IirSum& mix, int c, uint32_t tmem, bool to_strip) {
     const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads, last = n - 1;
@@ -430,7 +431,8 @@ __device__ __forceinline__ void strip_sum(float* strip, int n, const IirSum& mix
     uint32_t taddr = tmem + (uint32_t(32 * (warp & 3)) << 16) + 4u * uint32_t(warp >> 2);
     for (int q0 = 32 * warp, row = int(threadIdx.x) / kQuads; q0 < kQuads * n; q0 += kColThreads, row += kQuadRows, taddr += 12u) {
         float4* at = reinterpret_cast<float4*>(strip + size_t(min(row, last)) * kColLines + 4 * qd);
-        const float4 a = sum_quad<MULTI>(wc, *at, c == 0, taddr);
+        const float4 v = row <= last ? *at : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 a = sum_quad<MULTI>(wc, v, c == 0, taddr);
         if (MULTI && !to_strip) tmem_st4(taddr, a);
         else if (row <= last) *at = a;
     }
