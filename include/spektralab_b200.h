@@ -113,6 +113,10 @@ SPK_API spk_status spkx_philox(const uint32_t* counters, const uint32_t* keys, u
  * SPK_ERR_GPU with the context still usable. Process-wide; set it back to 0 afterwards. */
 SPK_API spk_status spkx_test_set_tc_wait_limit(int64_t cycles);
 
+/* Test hook of the paths taken when device memory is short: the session's frame, tier images, negatives and scratch
+ * together are refused more than `bytes` (0: no limit), as a device without more memory would refuse them. */
+SPK_API spk_status spkx_test_set_scratch_limit(spk_session* session, uint64_t bytes);
+
 /* Test hooks of the recursive blur's column pass (no counterpart in the reference engine), which loads its
  * strips by TMA and waits on an mbarrier. spkx_test_set_iir_wait_limit: the SM clocks a strip wait may
  * take before it gives up (0: the normal limit, about 2 s; process-wide, set it back to 0 afterwards). A

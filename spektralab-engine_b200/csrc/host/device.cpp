@@ -18,6 +18,7 @@ struct PoolState {
     std::mutex m;
     cudaStream_t stream = nullptr;
     size_t live = 0;
+    size_t limit = 0;
 };
 
 namespace {
@@ -67,8 +68,17 @@ void Pool::set_stream(cudaStream_t s) {
 
 cudaStream_t Pool::stream() const { return s_->stream; }
 
-DevBuffer Pool::acquire(size_t bytes) {
+void Pool::set_limit(size_t bytes) {
+    std::lock_guard<std::mutex> g(s_->m);
+    s_->limit = bytes;
+}
+
+cudaError_t Pool::allocate(size_t bytes, DevBuffer& b) {
     bytes = std::max<size_t>((bytes + 255) / 256 * 256, 256);
+    {
+        std::lock_guard<std::mutex> g(s_->m);
+        if (s_->limit && s_->live + bytes > s_->limit) return cudaErrorMemoryAllocation;
+    }
     void* p = nullptr;
     cudaError_t e = cudaMallocAsync(&p, bytes, s_->stream);
     if (e != cudaSuccess) {
@@ -77,7 +87,8 @@ DevBuffer Pool::acquire(size_t bytes) {
         cudaGetDevice(&dev);
         cudaStreamSynchronize(s_->stream);
         device_pool_trim(dev);
-        cuda_check(cudaMallocAsync(&p, bytes, s_->stream), "cudaMallocAsync (scratch)");
+        e = cudaMallocAsync(&p, bytes, s_->stream);
+        if (e != cudaSuccess) return e;
     }
     {
         std::lock_guard<std::mutex> g(s_->m);
@@ -89,8 +100,19 @@ DevBuffer Pool::acquire(size_t bytes) {
     impl->p = p;
     impl->size = bytes;
     impl->pool = s_;
-    DevBuffer b;
     b.p_ = std::move(impl);
+    return cudaSuccess;
+}
+
+DevBuffer Pool::acquire(size_t bytes) {
+    DevBuffer b;
+    cuda_check(allocate(bytes, b), "cudaMallocAsync (scratch)");
+    return b;
+}
+
+DevBuffer Pool::try_acquire(size_t bytes) {
+    DevBuffer b;
+    if (allocate(bytes, b) != cudaSuccess) (void)cudaGetLastError();
     return b;
 }
 

@@ -48,10 +48,13 @@ public:
     void set_stream(cudaStream_t s);
     cudaStream_t stream() const;
     DevBuffer acquire(size_t bytes);          // stream-ordered device memory, contents undefined
+    DevBuffer try_acquire(size_t bytes);      // the same; empty when the memory is not to be had
     DevBuffer persistent(size_t bytes);       // cudaMalloc'd: may outlive the stream
     size_t live_bytes() const;                // bytes of this pool's live scratch buffers
+    void set_limit(size_t bytes);             // test hook: live bytes refused above it, as by a full device (0: none)
 
 private:
+    cudaError_t allocate(size_t bytes, DevBuffer& b);
     std::shared_ptr<PoolState> s_;
 };
 
@@ -91,6 +94,11 @@ inline Plane make_plane(Pool& pool, uint32_t w, uint32_t h) {
     p.h = h;
     p.buf = pool.acquire(size_t(w) * h * 3 * sizeof(float));
     return p;
+}
+
+// The same; an empty plane when the memory is not to be had
+inline Plane try_plane(Pool& pool, uint32_t w, uint32_t h) {
+    return Plane{pool.try_acquire(size_t(w) * h * 3 * sizeof(float)), w, h};
 }
 
 // The result image behind spk_result.texture.

@@ -2627,6 +2627,14 @@ SPK_API spk_status spkx_test_set_tc_wait_limit(int64_t cycles) {
     return SPK_OK;
 }
 
+SPK_API spk_status spkx_test_set_scratch_limit(spk_session* session, uint64_t bytes) {
+    last_error::clear();
+    if (!session) return invalid("session is NULL");
+    std::lock_guard<std::mutex> lock(S(session)->m);
+    S(session)->pool.set_limit(size_t(bytes));
+    return SPK_OK;
+}
+
 SPK_API spk_status spkx_test_set_iir_wait_limit(int64_t cycles) {
     last_error::clear();
     if (cycles < 0) return invalid("a wait limit is a count of SM clocks, 0 or more");

@@ -382,14 +382,83 @@ void gaussian(RenderCtx& ctx, const Plane& in, const Plane& dst, const Vec3& sig
     encode_blur(ctx, in, dst, sigma, Fuse{});
 }
 
+namespace {
+bool all_fir(const MixtureComponent& m) {
+    return blur_branch(m.sigma[0]) != Branch::Iir && blur_branch(m.sigma[1]) != Branch::Iir &&
+           blur_branch(m.sigma[2]) != Branch::Iir;
+}
+
+// The components from k on that have a recursive channel, at most `limit`, added to acc (k = 0: acc starts with
+// them): the FIR channels of each first, then the row passes of all of them in one launch, the column passes
+// of those that also have FIR channels in another, and the sum in order (encode_blur's operations). A line
+// pass is as long as a line, and one component's lines leave most of the chip idle (three mixed components,
+// the whole halation joined and one by one: 0.50 and 1.07 ms at 1600 x 1067, 3.68 and 5.63 at 6000 x 4000).
+// Returns how many it took; 0, with nothing launched, when the planes of more than one are not to be had.
+size_t line_run(RenderCtx& ctx, const Plane& in, const Plane& acc, const std::vector<MixtureComponent>& comps, size_t k,
+                size_t limit) {
+    struct Component {
+        bool iir[3];
+        FirTaps fir_taps;
+        Plane fir, work, blurred;  // fir: of the FIR channels; blurred: of components that have any
+    };
+    std::vector<Component> run;
+    const auto plane = [&](Plane& p) {
+        p = limit > 1 ? try_plane(ctx.pool, in.w, in.h) : make_plane(ctx.pool, in.w, in.h);
+        return static_cast<bool>(p);
+    };
+    for (size_t j = k; j < comps.size() && run.size() < limit && !all_fir(comps[j]); ++j) {
+        Component& m = run.emplace_back();
+        int n_iir = 0;
+        for (int c = 0; c < 3; ++c) {
+            m.iir[c] = blur_branch(comps[j].sigma[c]) == Branch::Iir;
+            n_iir += m.iir[c];
+        }
+        m.fir_taps = fir_taps(comps[j].sigma, m.iir);
+        if (n_iir < 3 && m.fir_taps.r > 0 && !plane(m.fir)) return 0;
+        if (!plane(m.work) || (n_iir < 3 && !plane(m.blurred))) return 0;
+    }
+    IirLineJobs rows{}, cols{};
+    for (size_t i = 0; i < run.size(); ++i) {
+        Component& m = run[i];
+        if (m.fir) encode_fir(ctx, in, m.fir, m.fir_taps, Fuse{});
+        rows.in[rows.n] = m.fir ? m.fir.data() : in.data();
+        rows.work[rows.n] = m.work.data();
+        rows.q[rows.n] = iir_coefs(comps[k + i].sigma, m.iir);
+        if (m.blurred) {
+            cols.work[cols.n] = m.work.data();
+            cols.out[cols.n] = m.blurred.data();
+            cols.q[cols.n++] = rows.q[rows.n];
+        }
+        ++rows.n;
+    }
+    dev::iir_h_lines(rows, in.w, in.h, ctx.stream);
+    dev::iir_v_lines(cols, in.w, in.h, ctx.stream);
+    for (size_t i = 0; i < run.size(); ++i) {
+        const Vec3& weight = comps[k + i].weight;
+        const bool start = k + i == 0;
+        if (run[i].blurred) {
+            if (start) lincomb(ctx, weight, run[i].blurred, Vec3{1.0, 1.0, 1.0}, nullptr, acc);
+            else lincomb(ctx, Vec3{1.0, 1.0, 1.0}, acc, weight, &run[i].blurred, acc);
+        } else {
+            float wt[3];
+            weights(weight, wt);
+            dev::iir_v(run[i].work.data(), acc.data(), acc.data(), in.w, in.h, rows.q[i], start ? ACC_ZERO : ACC_PLANE, wt,
+                       ctx.stream);
+        }
+    }
+    return run.size();
+}
+}  // namespace
+
 void gaussian_mixture(RenderCtx& ctx, const Plane& in, const Plane& out, const std::vector<MixtureComponent>& comps) {
     if (comps.empty()) fail_internal("empty mixture");
     Plane acc = same(in, out) ? make_plane(ctx.pool, in.w, in.h) : out;
     const bool no_iir[3] = {false, false, false};
-    const auto all_fir = [](const MixtureComponent& m) {
-        return blur_branch(m.sigma[0]) != Branch::Iir && blur_branch(m.sigma[1]) != Branch::Iir &&
-               blur_branch(m.sigma[2]) != Branch::Iir;
-    };
+    // A run holds up to three planes of 12 bytes a pixel per component: they are kept within 4 GiB, and frames
+    // above 60 megapixels take one component at a time.
+    constexpr uint64_t kRunBytes = uint64_t(4) << 30;
+    const uint64_t limit = std::clamp<uint64_t>(kRunBytes / (36 * std::max<uint64_t>(in.pixels(), 1)), 1,
+                                                SPKB_MAX_COMPONENTS);
     for (size_t k = 0; k < comps.size(); ++k) {
         const MixtureComponent& m = comps[k];
         const bool ident = !(m.sigma[0] > 0.0) && !(m.sigma[1] > 0.0) && !(m.sigma[2] > 0.0);
@@ -420,60 +489,10 @@ void gaussian_mixture(RenderCtx& ctx, const Plane& in, const Plane& out, const s
             encode_blur(ctx, in, acc, m.sigma, f);
             continue;
         }
-        // a run of components with a recursive channel: the FIR channels of each first, then the row passes of
-        // all of them in one launch, the column passes of those that also have FIR channels in another, and
-        // the sum in order (encode_blur's operations). A line pass is as long as a line, and one component's
-        // lines leave most of the chip idle (three mixed components, the whole halation joined and one by one:
-        // 0.50 and 1.07 ms at 1600 x 1067, 3.68 and 5.63 at 6000 x 4000). A run holds up to three planes of 12
-        // bytes a pixel per component: they are kept within 4 GiB, and frames above 60 megapixels take one
-        // component at a time.
-        constexpr uint64_t kRunBytes = uint64_t(4) << 30;
-        const uint64_t limit = std::clamp<uint64_t>(kRunBytes / (36 * std::max<uint64_t>(in.pixels(), 1)), 1,
-                                                    SPKB_MAX_COMPONENTS);
-        std::vector<Plane> fir, work, blurred;
-        IirLineJobs rows{}, cols{};
-        for (j = k; j < comps.size() && rows.n < limit && !all_fir(comps[j]); ++j) {
-            bool iir[3];
-            int n_iir = 0;
-            for (int c = 0; c < 3; ++c) {
-                iir[c] = blur_branch(comps[j].sigma[c]) == Branch::Iir;
-                n_iir += iir[c];
-            }
-            const FirTaps fa = fir_taps(comps[j].sigma, iir);
-            const float* src = in.data();
-            if (n_iir < 3 && fa.r > 0) {
-                fir.push_back(make_plane(ctx.pool, in.w, in.h));
-                encode_fir(ctx, in, fir.back(), fa, Fuse{});
-                src = fir.back().data();
-            }
-            work.push_back(make_plane(ctx.pool, in.w, in.h));
-            blurred.push_back(n_iir < 3 ? make_plane(ctx.pool, in.w, in.h) : Plane{});
-            rows.in[rows.n] = src;
-            rows.work[rows.n] = work.back().data();
-            rows.q[rows.n] = iir_coefs(comps[j].sigma, iir);
-            if (n_iir < 3) {
-                cols.work[cols.n] = work.back().data();
-                cols.out[cols.n] = blurred.back().data();
-                cols.q[cols.n++] = rows.q[rows.n];
-            }
-            ++rows.n;
-        }
-        dev::iir_h_lines(rows, in.w, in.h, ctx.stream);
-        dev::iir_v_lines(cols, in.w, in.h, ctx.stream);
-        for (size_t i = 0; i < rows.n; ++i) {
-            const MixtureComponent& mi = comps[k + i];
-            const bool start = k + i == 0;
-            if (blurred[i]) {
-                if (start) lincomb(ctx, mi.weight, blurred[i], Vec3{1.0, 1.0, 1.0}, nullptr, acc);
-                else lincomb(ctx, Vec3{1.0, 1.0, 1.0}, acc, mi.weight, &blurred[i], acc);
-            } else {
-                float wt[3];
-                weights(mi.weight, wt);
-                dev::iir_v(work[i].data(), acc.data(), acc.data(), in.w, in.h, rows.q[i], start ? ACC_ZERO : ACC_PLANE, wt,
-                           ctx.stream);
-            }
-        }
-        k = j - 1;
+        // a run of components with a recursive channel, or one at a time when its planes are not to be had
+        size_t taken = line_run(ctx, in, acc, comps, k, limit);
+        if (taken == 0) taken = line_run(ctx, in, acc, comps, k, 1);
+        k += taken - 1;
     }
     if (!same(acc, out)) dev::copy(acc.data(), out.data(), acc.pixels(), ctx.stream);
 }

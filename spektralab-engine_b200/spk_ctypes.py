@@ -110,6 +110,7 @@ EXT = {
     "spkx_session_set_print_mode": (I32, [P, C, U32]),
     "spkx_print_negative": (I32, [P, P, U32, U32, P, U32, P, ctypes.POINTER(ctypes.c_double)]),
     "spkx_test_set_tc_wait_limit": (I32, [ctypes.c_int64]),
+    "spkx_test_set_scratch_limit": (I32, [P, ctypes.c_uint64]),
     "spkx_test_set_iir_wait_limit": (I32, [ctypes.c_int64]),
     "spkx_test_take_iir_waits_given_up": (I32, [UP]),
 }
@@ -400,6 +401,10 @@ class Session:
     def set_print_mode(self, mode, bins=81):
         """spkx_session_set_print_mode: fp32, fp32_generic, fp64, tf32, bf16 or bf16x3 at 81 or 401 wavelengths."""
         self.L.check(self.L.lib.spkx_session_set_print_mode(self.h, mode.encode(), bins))
+
+    def set_scratch_limit(self, nbytes):
+        """spkx_test_set_scratch_limit: device memory of this session beyond nbytes is refused (0: no limit)."""
+        self.L.check(self.L.lib.spkx_test_set_scratch_limit(self.h, nbytes))
 
     def print_negative(self, negative_ptr, width, height, rgba16_ptr, row_stride_px, contraction_ptr=None):
         """spkx_print_negative on device pointers (ints); returns the print kernel's device time in ms."""
