@@ -577,7 +577,8 @@ void render(Session& s, const char* tier_name, bool reprint, spk_result* out) {
         }
         ctx.print_seed = s.draw_print_seed();
         ctx.pitch_um = ts.pitch_um;
-        img = output_acquire(s.engine->device, ts.negative.w, ts.negative.h);
+        with_film_memory(ctx, ts.negative.h,
+                         [&] { img = output_acquire(s.engine->device, ts.negative.w, ts.negative.h); });
         ctx.copy_stream = s.copy_stream;
         ctx.band_events = &s.band_events;
         if (!print_scan_encode(ctx, s.pipe, s.live, ts.negative, img, true))

@@ -1237,17 +1237,31 @@ void print_nodes(RenderCtx& ctx, const PrintSetup& s) {
     print_nodes_tail(ctx, s);
 }
 
+bool RenderCtx::release_film(uint32_t h) {
+    if (!film_rows) return false;
+    film_rows(h);
+    film_rows = nullptr;
+    // an allocation outside the pool gets the planes only once they are freed and given back
+    int device = 0;
+    cuda_check(cudaStreamSynchronize(stream), "film");
+    cuda_check(cudaGetDevice(&device), "cudaGetDevice");
+    device_pool_trim(device);
+    return true;
+}
+
 bool print_scan_encode(RenderCtx& ctx, const Pipeline& p, const LiveParams& live, const Plane& negative,
                        OutputImage* img, bool to_host) {
     const PrintSetup& s = *p.print;
     print_nodes_head(ctx, s);
     const uint32_t w = negative.w, h = negative.h;
-    Plane rgb = make_plane(ctx.pool, w, h);
-    Plane glare;
-    if (!s.scanned && s.glare_draws()) {
-        Stage st(ctx, "glare");
-        glare = glare_plane(ctx, p, w, h);
-    }
+    Plane rgb, glare;
+    with_film_memory(ctx, h, [&] {
+        if (!rgb) rgb = make_plane(ctx.pool, w, h);
+        if (!s.scanned && s.glare_draws()) {
+            Stage st(ctx, "glare");
+            glare = glare_plane(ctx, p, w, h);
+        }
+    });
     const float* gl = glare ? glare.data() : nullptr;
     ScanArgs sa;
     const bool tiled = scan_args(p, ctx.rho_tier, w, h, img->stride_px, sa);

@@ -14,6 +14,7 @@
 #include "../cuda/launch.hpp"
 #include "device.hpp"
 #include "setup.hpp"
+#include "status.hpp"
 
 namespace spkb {
 
@@ -92,7 +93,22 @@ struct RenderCtx {
     // the last rows are drawn. print_scan_encode calls it; the planes it holds live as long as it does.
     bool defer_grain = false;
     std::function<void(uint32_t n)> film_rows = nullptr;
+    // the whole negative drawn and the planes that film_rows held freed, when memory is short; false: none were held
+    bool release_film(uint32_t h);
 };
+
+// f(), which takes device memory for the print of a negative of h rows: again with the film's planes freed when
+// the memory is short and they are still held
+template <class F>
+void with_film_memory(RenderCtx& ctx, uint32_t h, F&& f) {
+    try {
+        f();
+        return;
+    } catch (const Error& e) {
+        if (e.status() != SPK_ERR_GPU || !ctx.release_film(h)) throw;
+    }
+    f();
+}
 
 // Stage timing with CUDA events on the render stream (bench and profile entry points).
 struct Timer : dev::LaunchHook {

@@ -9,11 +9,29 @@ from conftest import BASE, sc
 pytestmark = pytest.mark.gpu
 
 MIXED = [((0.1, 0.2, 0.3), (3.0 + 0.5 * k, 0.4 * k + 0.3, 4.0)) for k in range(6)]
+FIRST_SEED = 0x4ABEA221  # of a session's first develop
 SLACK = 1 << 18  # tables and rounding: less than a plane of the frames below
 
 
 def plane(w, h):
     return 12 * w * h
+
+
+def test_grain_in_bands_released_for_the_print(engine):
+    """A frame whose grain is drawn in bands holds the exposure and grain planes through the print. The frame, the
+    negative, the print's output and the glare's two planes fit; with those two they do not."""
+    w, h = 2048, 2100
+    delta = dict(BASE, halation_active=False, glare_active=True, film_format_mm=0.009 * h)  # a pitch of 9 um
+    img = sc.synthetic_image(w, h, 2)
+    with engine.open(img, delta) as s:
+        want = s.render("full")[0].copy()
+    for planes in (5, 6, 7):
+        with engine.open(img, delta) as s:
+            s.set_scratch_limit(planes * plane(w, h) + SLACK)
+            np.testing.assert_array_equal(s.render("full")[0], want)
+            s.set_scratch_limit(0)
+            negative = s.negative("full", w, h)
+            np.testing.assert_array_equal(negative, s.develop_debug("full", FIRST_SEED, w, h, counts=False)[0])
 
 
 def test_mixed_components_one_at_a_time(engine):
