@@ -117,6 +117,9 @@ SPK_API spk_status spkx_test_set_tc_wait_limit(int64_t cycles);
  * together are refused more than `bytes` (0: no limit), as a device without more memory would refuse them. */
 SPK_API spk_status spkx_test_set_scratch_limit(spk_session* session, uint64_t bytes);
 
+/* The kernels that this library has launched since it was loaded (process-wide; graph replays not counted). */
+SPK_API spk_status spkx_test_launch_count(uint64_t* count);
+
 /* Test hooks of the recursive blur's column pass (no counterpart in the reference engine), which loads its
  * strips by TMA and waits on an mbarrier. spkx_test_set_iir_wait_limit: the SM clocks a strip wait may
  * take before it gives up (0: the normal limit, about 2 s; process-wide, set it back to 0 afterwards). A

@@ -570,6 +570,8 @@ void render(Session& s, const char* tier_name, bool reprint, spk_result* out) {
         ctx.rho_tier = s.rho(ts);
         ctx.print_mode = s.print_mode;
         ctx.print_bins = s.print_bins;
+        ctx.copy_stream = s.copy_stream;
+        ctx.band_events = &s.band_events;
         if (!reuse) {
             developed = true;
             ctx.defer_grain = true;
@@ -579,8 +581,6 @@ void render(Session& s, const char* tier_name, bool reprint, spk_result* out) {
         ctx.pitch_um = ts.pitch_um;
         with_film_memory(ctx, ts.negative.h,
                          [&] { img = output_acquire(s.engine->device, ts.negative.w, ts.negative.h); });
-        ctx.copy_stream = s.copy_stream;
-        ctx.band_events = &s.band_events;
         if (!print_scan_encode(ctx, s.pipe, s.live, ts.negative, img, true))
             cuda_check(cudaMemcpyAsync(img->host, img->dev, img->bytes, cudaMemcpyDeviceToHost, s.stream),
                        "result copy");
@@ -2633,6 +2633,13 @@ SPK_API spk_status spkx_test_set_scratch_limit(spk_session* session, uint64_t by
     if (!session) return invalid("session is NULL");
     std::lock_guard<std::mutex> lock(S(session)->m);
     S(session)->pool.set_limit(size_t(bytes));
+    return SPK_OK;
+}
+
+SPK_API spk_status spkx_test_launch_count(uint64_t* count) {
+    last_error::clear();
+    if (!count) return invalid("count is NULL");
+    *count = dev::launch_count();
     return SPK_OK;
 }
 

@@ -830,6 +830,14 @@ constexpr uint32_t kBandRows = 8 * dev::scan_tile_rows();  // of the print side'
 // the print, up to 36 bytes a pixel (2.3 GB) more scratch at once than a frame drawn whole: hence the upper end.
 constexpr size_t kDeferFrom = size_t(4) << 20, kDeferTo = size_t(64) << 20;
 
+namespace {
+// Whether print_scan_encode, asked for a copy on the host, prints a negative of h rows in bands; tiled: scan_args
+// takes the frame
+bool print_in_bands(const RenderCtx& ctx, bool tiled, uint32_t h) {
+    return tiled && ctx.print_mode < 0 && ctx.copy_stream && ctx.band_events && h > kBandRows;
+}
+}  // namespace
+
 Plane develop(RenderCtx& ctx, const Pipeline& p, const Plane& tier_source, uint32_t film_seed,
               const std::optional<HalationOverride>& hov, float* counts_out, float* lam_out) {
     const FilmSetup& f = *p.film;
@@ -901,11 +909,12 @@ Plane develop(RenderCtx& ctx, const Pipeline& p, const Plane& tier_source, uint3
     }
     Plane G = make_plane(ctx.pool, w, h);
     if (ctx.defer_grain && dp.amount == 1.0 && da.grain && da.mode == 0 && dp.final_blur > 0.0 &&
-        blur_branch(dp.final_blur) == Branch::Fir && h > kBandRows && source.pixels() >= kDeferFrom &&
-        source.pixels() <= kDeferTo) {
+        blur_branch(dp.final_blur) == Branch::Fir && source.pixels() >= kDeferFrom && source.pixels() <= kDeferTo) {
         const bool no_iir[3] = {false, false, false};
         const FirTaps t = fir_taps(Vec3{dp.final_blur, dp.final_blur, dp.final_blur}, no_iir);
-        if (t.r > 0 && uniform_taps(t) && dev::fir_tile_fits(w, h, t.r)) {
+        ScanArgs sa;
+        if (t.r > 0 && uniform_taps(t) && dev::fir_tile_fits(w, h, t.r) &&
+            print_in_bands(ctx, scan_args(p, ctx.rho_tier, w, h, 0, sa), h)) {
             ctx.film_rows = [=, stream = ctx.stream, drawn = 0u, blurred = 0u](uint32_t n) mutable {
                 const uint32_t tiles = (std::min(n, h) + dev::kFirTileRows - 1) / dev::kFirTileRows;
                 const uint32_t b = std::min(h, tiles * dev::kFirTileRows), d = std::min(h, b + uint32_t(t.r));
@@ -1265,13 +1274,12 @@ bool print_scan_encode(RenderCtx& ctx, const Pipeline& p, const LiveParams& live
     const float* gl = glare ? glare.data() : nullptr;
     ScanArgs sa;
     const bool tiled = scan_args(p, ctx.rho_tier, w, h, img->stride_px, sa);
-    if (to_host && tiled && ctx.print_mode < 0 && ctx.copy_stream && ctx.band_events && h > kBandRows) {
+    if (to_host && print_in_bands(ctx, tiled, h)) {
         print_nodes_tail(ctx, s);
         Stage st(ctx, "print_scanner");
         print_scan_banded(ctx, p, live, negative, rgb, img, sa, gl);
         return true;
     }
-    if (ctx.film_rows) ctx.film_rows(h);
     {
         Stage st(ctx, "print");
         print_stage(ctx, p, live, negative, rgb, gl);

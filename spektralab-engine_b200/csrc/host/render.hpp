@@ -88,9 +88,10 @@ struct RenderCtx {
     // band_events, grown as needed), overlapping the next band's kernels; null: no banded copy
     cudaStream_t copy_stream = nullptr;
     std::vector<cudaEvent_t>* band_events = nullptr;
-    // defer_grain: develop() may leave the grain draws and their blur to film_rows, which enqueues the negative's
-    // rows below n (calls with rising n), so that the print's bands, and the copies of their results, start before
-    // the last rows are drawn. print_scan_encode calls it; the planes it holds live as long as it does.
+    // defer_grain: print_scan_encode with a copy on the host follows in this context. Where it prints in bands,
+    // develop() may leave the grain draws and their blur to film_rows, which enqueues the negative's rows below n
+    // (calls with rising n), so that the bands, and the copies of their results, start before the last rows are
+    // drawn. The bands call it; the planes it holds live as long as it does.
     bool defer_grain = false;
     std::function<void(uint32_t n)> film_rows = nullptr;
     // the whole negative drawn and the planes that film_rows held freed, when memory is short; false: none were held
