@@ -69,28 +69,33 @@ Plane downscale(Pool& pool, cudaStream_t s, const Plane& src, uint32_t long_edge
     cuda_check(cudaMemcpyAsync(tab.ptr(), words.data(), words.size() * 4, cudaMemcpyHostToDevice, s), "tier tables");
     const uint32_t* base = tab.as<uint32_t>();
 
-    const uint32_t* yi = base + oyi;
-    Plane v = src;
-    if (ty.size() > 1) {  // the vertically filtered rows that the samples read, in the samples' order
-        v = make_plane(pool, src.w, 2 * o.h);
-        TierBlurArgs a{reinterpret_cast<const float*>(base + oty), yi, src.w, src.h, o.h, int32_t(ty.size() / 2)};
-        dev::tier_rows(src.data(), v.data(), a, s);
-        yi = nullptr;
-    }
     // from the session's stream-ordered pool, as the frame itself: cudaMalloc and cudaFree would stop the device
     // in every open and close
     Plane out = make_plane(pool, o.w, o.h);
-    TierResampleArgs r{};
-    r.taps_x = reinterpret_cast<const float*>(base + otx);
-    r.xi = base + oxi;
-    r.xt = reinterpret_cast<const float*>(base + oxt);
-    r.yi = yi;
-    r.yt = reinterpret_cast<const float*>(base + oyt);
-    r.in_w = src.w;
-    r.out_w = o.w;
-    r.out_h = o.h;
-    r.rx = int32_t(tx.size() / 2);
-    dev::tier_resample(v.data(), out.data(), r, s);
+    // The vertically filtered rows that the samples read, in the samples' order, two per output row: in two
+    // halves where all of them would take more than the frame itself
+    const bool filter = ty.size() > 1;
+    const uint32_t part = filter && 2 * uint64_t(o.h) > src.h ? (o.h + 1) / 2 : o.h;
+    Plane v = filter ? make_plane(pool, src.w, 2 * part) : src;
+    for (uint32_t y = 0; y < o.h; y += part) {
+        const uint32_t rows = std::min(part, o.h - y);
+        const uint32_t* yi = base + oyi + 2 * size_t(y);
+        if (filter) {
+            TierBlurArgs a{reinterpret_cast<const float*>(base + oty), yi, src.w, src.h, rows, int32_t(ty.size() / 2)};
+            dev::tier_rows(src.data(), v.data(), a, s);
+        }
+        TierResampleArgs r{};
+        r.taps_x = reinterpret_cast<const float*>(base + otx);
+        r.xi = base + oxi;
+        r.xt = reinterpret_cast<const float*>(base + oxt);
+        r.yi = filter ? nullptr : yi;
+        r.yt = reinterpret_cast<const float*>(base + oyt) + y;
+        r.in_w = src.w;
+        r.out_w = o.w;
+        r.out_h = rows;
+        r.rx = int32_t(tx.size() / 2);
+        dev::tier_resample(v.data(), out.data() + 3 * size_t(y) * o.w, r, s);
+    }
     cuda_check(cudaStreamSynchronize(s), "tier downscale");  // the host tables go out of scope
     return out;
 }

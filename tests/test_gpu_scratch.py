@@ -4,6 +4,7 @@ falls back to that one and gives the same bits. The session's limit stands in fo
 import numpy as np
 import pytest
 
+import oracle
 from conftest import BASE, sc
 
 pytestmark = pytest.mark.gpu
@@ -32,6 +33,21 @@ def test_grain_in_bands_released_for_the_print(engine):
             s.set_scratch_limit(0)
             negative = s.negative("full", w, h)
             np.testing.assert_array_equal(negative, s.develop_debug("full", FIRST_SEED, w, h, counts=False)[0])
+
+
+@pytest.mark.parametrize("w,h,tier", [(4421, 300, "preview"), (6601, 201, "preview"), (1001, 1301, "live")])
+def test_tier_image_beside_the_frame(engine, w, h, tier):
+    """A tier not much smaller than the frame: the tier's image and one more plane of the frame's size fit beside the
+    frame, the two filtered rows per output row together would not."""
+    img = sc.synthetic_image(w, h, 3)
+    delta = dict(BASE, preview_long_edge=800)
+    with engine.open(img, delta) as s:
+        want = s.tier_image(tier)
+    np.testing.assert_array_equal(want, oracle.downscale(img, 3400 if tier == "preview" else 800))
+    assert h / 2 < want.shape[0] <= h / 1.25  # a ratio that has a filter
+    with engine.open(img, delta) as s:
+        s.set_scratch_limit(2 * plane(w, h) + want.nbytes + SLACK)
+        np.testing.assert_array_equal(s.tier_image(tier), want)
 
 
 def test_mixed_components_one_at_a_time(engine):
