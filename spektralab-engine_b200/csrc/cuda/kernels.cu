@@ -37,91 +37,11 @@ __device__ __forceinline__ float mitchell(float u) {
     return 0.0f;
 }
 
-__device__ __forceinline__ void mitchell_axis(float t, uint32_t L, int* idx, float* w) {
-    const float last = float(L - 1);
-    float u = t * last;
-    int base;
-    float frac;
-    if (u <= 0.0f) u = 0.0f;
-    if (u >= last) {
-        base = int(L) - 2;
-        frac = 1.0f;
-    } else {
-        base = int(floorf(u));
-        frac = u - float(base);
-    }
-    const int n = int(L);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        int i = base - 1 + k;
-        if (i < 0) i = -i;
-        if (i >= n) i = 2 * (n - 1) - i;
-        idx[k] = i;
-    }
-    w[0] = mitchell(frac + 1.0f);
-    w[1] = mitchell(frac);
-    w[2] = mitchell(frac - 1.0f);
-    w[3] = mitchell(frac - 2.0f);
-}
-
-__global__ void k_expose(const float* __restrict__ rgb, float* __restrict__ hout, const float4* __restrict__ table,
-                         const __grid_constant__ ExposeArgs q) {
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= q.n) return;
-    float r = rgb[3 * size_t(gid)], g = rgb[3 * size_t(gid) + 1], b = rgb[3 * size_t(gid) + 2];
-    if (q.apply_ae) {  // the auto-exposure scale pass (reference src/film/develop.cpp:132-140), one rounding each
-        r = __fmul_rn(r, q.ae_gain);
-        g = __fmul_rn(g, q.ae_gain);
-        b = __fmul_rn(b, q.ae_gain);
-    }
-    const float X = (q.a[0] * r + q.a[1] * g) + q.a[2] * b;
-    const float Y = (q.a[3] * r + q.a[4] * g) + q.a[5] * b;
-    const float Z = (q.a[6] * r + q.a[7] * g) + q.a[8] * b;
-    const float bs = (X + Y) + Z;
-    const float d = bs > 1e-10f ? bs : 1e-10f;
-    const float x = X / d, y = Y / d, o = 1.0f - x;
-    const float t0 = fminf(fmaxf(o * o, 0.0f), 1.0f);
-    const float t1 = fminf(fmaxf(y / (o > 1e-10f ? o : 1e-10f), 0.0f), 1.0f);
-    const float bp = isnan(bs) ? 0.0f : bs;
-    int ia[4], ib[4];
-    float wa[4], wb[4];
-    mitchell_axis(t0, q.L, ia, wa);
-    mitchell_axis(t1, q.L, ib, wb);
-    float s = 0.0f, a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float w = wa[i] * wb[j];
-            const float4 t = __ldg(table + (size_t(ia[i]) * q.L + size_t(ib[j])));
-            s += w;
-            a0 += w * t.x;
-            a1 += w * t.y;
-            a2 += w * t.z;
-        }
-    }
-    if (s != 0.0f) {
-        a0 = a0 / s;
-        a1 = a1 / s;
-        a2 = a2 / s;
-    }
-    float h0 = bp * a0, h1 = bp * a1, h2 = bp * a2;
-    if (q.apply_gain) {
-        h0 = h0 * q.gain;
-        h1 = h1 * q.gain;
-        h2 = h2 * q.gain;
-    }
-    hout[3 * size_t(gid)] = h0;
-    hout[3 * size_t(gid) + 1] = h1;
-    hout[3 * size_t(gid) + 2] = h2;
-}
-
-// The same pass over a table of 4 x 4 patches. Patch (ba, bb) holds the sixteen texels the bicubic reads
-// when the pixel's base indices are (ba, bb) -- row reflect(ba - 1 + i), column reflect(bb - 1 + j) -- as
-// RGB triples in the loop order (i outer, j inner): 48 floats, 192 bytes, fetched with six 32-byte loads
-// instead of sixteen 16-byte gathers, so a warp's random lookups take about a third of the L1 wavefronts.
-// The arithmetic is k_expose's, operation for operation. One pixel per thread: a thread's lookups wait on its
-// divisions, so pixels in turn in one thread only add up their waits.
+// The table comes as 4 x 4 patches. Patch (ba, bb) holds the sixteen texels the bicubic reads when the
+// pixel's base indices are (ba, bb) -- row reflect(ba - 1 + i), column reflect(bb - 1 + j) -- as RGB triples
+// in the loop order (i outer, j inner): 48 floats, 192 bytes, fetched with six 32-byte loads instead of
+// sixteen 16-byte gathers, so a warp's random lookups take about a third of the L1 wavefronts. One pixel per
+// thread: a thread's lookups wait on its divisions, so pixels in turn in one thread only add up their waits.
 
 __device__ __forceinline__ void mitchell_base(float t, uint32_t L, int& base, float w[4]) {
     const float last = float(L - 1);
@@ -1406,15 +1326,10 @@ void ensure_smem(const void* kernel, int bytes) {
 void set_launch_hook(LaunchHook* hook) { t_hook = hook; }
 uint64_t launch_count() { return g_launches.load(); }
 
-void expose(const float* rgb, float* h, const float* table4, const float* patches, const ExposeArgs& a,
-            cudaStream_t s) {
+void expose(const float* rgb, float* h, const float* patches, const ExposeArgs& a, cudaStream_t s) {
     if (a.n == 0) return;
     Probe p("expose", s);
-    if (patches) {
-        k_expose_patch<<<div_up(a.n, kExposeThreads), kExposeThreads, 0, s>>>(rgb, h, patches, a);
-        return;
-    }
-    k_expose<<<div_up(a.n, 256), 256, 0, s>>>(rgb, h, reinterpret_cast<const float4*>(table4), a);
+    k_expose_patch<<<div_up(a.n, kExposeThreads), kExposeThreads, 0, s>>>(rgb, h, patches, a);
 }
 
 void iir_tangent(const float* in, const float* in_dot, float* work, float* work_dot, float* out, float* out_dot,
