@@ -293,13 +293,11 @@ void encode_fir(RenderCtx& ctx, const Plane& in, const Plane& dst, const FirTaps
     dev::fir_h(tmp.data(), dst.data(), acc.data(), in.w, in.h, t, fuse.mode, w, ctx.stream);
 }
 
-void encode_iir(RenderCtx& ctx, const Plane& in, const Plane& dst, const IirCoefs& c, const Fuse& fuse) {
+void encode_iir(RenderCtx& ctx, const Plane& in, const Plane& dst, const IirCoefs& c) {
     Plane tmp = make_plane(ctx.pool, in.w, in.h);
     dev::iir_h(in.data(), tmp.data(), in.w, in.h, c, ctx.stream);
-    float w[3];
-    weights(fuse.weight, w);
-    const Plane& acc = (fuse.mode == ACC_PLANE && fuse.acc) ? *fuse.acc : dst;
-    dev::iir_v(tmp.data(), dst.data(), acc.data(), in.w, in.h, c, fuse.mode, w, ctx.stream);
+    const float one[3] = {1.0f, 1.0f, 1.0f};
+    dev::iir_v(tmp.data(), dst.data(), dst.data(), in.w, in.h, c, ACC_NONE, one, ctx.stream);
 }
 
 void lincomb(RenderCtx& ctx, const Vec3& a, const Plane& x, const Vec3& b, const Plane* y, const Plane& out) {
@@ -309,7 +307,7 @@ void lincomb(RenderCtx& ctx, const Vec3& a, const Plane& x, const Vec3& b, const
     dev::lincomb(x.data(), y ? y->data() : nullptr, out.data(), x.pixels(), fa, fb, ctx.stream);
 }
 
-void encode_blur(RenderCtx& ctx, const Plane& in, const Plane& dst, const Vec3& sigma, const Fuse& fuse) {
+void encode_blur(RenderCtx& ctx, const Plane& in, const Plane& dst, const Vec3& sigma) {
     bool iir[3];
     int n_iir = 0;
     for (int c = 0; c < 3; ++c) {
@@ -317,32 +315,16 @@ void encode_blur(RenderCtx& ctx, const Plane& in, const Plane& dst, const Vec3& 
         n_iir += iir[c];
     }
     const FirTaps fa = fir_taps(sigma, iir);
-    if (n_iir == 0) {
-        if (fuse.mode == ACC_NONE && fa.r == 0) {
-            if (!same(in, dst)) dev::copy(in.data(), dst.data(), in.pixels(), ctx.stream);
-            return;
-        }
-        encode_fir(ctx, in, dst, fa, fuse);
-        return;
-    }
-    const IirCoefs ia = iir_coefs(sigma, iir);
-    if (n_iir == 3) {
-        encode_iir(ctx, in, dst, ia, fuse);
-        return;
-    }
-    if (fuse.mode != ACC_NONE) {
-        Plane t = make_plane(ctx.pool, in.w, in.h);
-        encode_blur(ctx, in, t, sigma, Fuse{});
-        if (fuse.mode == ACC_ZERO) lincomb(ctx, fuse.weight, t, Vec3{1.0, 1.0, 1.0}, nullptr, dst);
-        else lincomb(ctx, Vec3{1.0, 1.0, 1.0}, *fuse.acc, fuse.weight, &t, dst);
-        return;
-    }
-    if (fa.r > 0) {
+    if (n_iir == 0 && fa.r == 0) {
+        if (!same(in, dst)) dev::copy(in.data(), dst.data(), in.pixels(), ctx.stream);
+    } else if (n_iir == 0) {
+        encode_fir(ctx, in, dst, fa, Fuse{});
+    } else if (n_iir < 3 && fa.r > 0) {
         Plane t = make_plane(ctx.pool, in.w, in.h);
         encode_fir(ctx, in, t, fa, Fuse{});
-        encode_iir(ctx, t, dst, ia, Fuse{});
+        encode_iir(ctx, t, dst, iir_coefs(sigma, iir));
     } else {
-        encode_iir(ctx, in, dst, ia, Fuse{});
+        encode_iir(ctx, in, dst, iir_coefs(sigma, iir));
     }
 }
 
@@ -379,7 +361,7 @@ void gaussian(RenderCtx& ctx, const Plane& in, const Plane& dst, const Vec3& sig
         Plane tmp = make_plane(ctx.pool, dev::iir_pitch(in.w), in.h);
         if (blur_iir_block(in.data(), dst.data(), tmp.data(), tmp.w, in.w, in.h, s3, all, ctx.stream)) return;
     }
-    encode_blur(ctx, in, dst, sigma, Fuse{});
+    encode_blur(ctx, in, dst, sigma);
 }
 
 namespace {
@@ -390,7 +372,7 @@ bool all_fir(const MixtureComponent& m) {
 
 // The components from k on that have a recursive channel, at most `limit`, added to acc (k = 0: acc starts with
 // them): the FIR channels of each first, then the row passes of all of them in one launch, the column passes
-// of those that also have FIR channels in another, and the sum in order (encode_blur's operations). A line
+// of those that also have FIR channels in another, and the sum in order (out = 0 + w v, then acc + w v). A line
 // pass is as long as a line, and one component's lines leave most of the chip idle (three mixed components,
 // the whole halation joined and one by one: 0.50 and 1.07 ms at 1600 x 1067, 3.68 and 5.63 at 6000 x 4000).
 // Returns how many it took; 0, with nothing launched, when the planes of more than one are not to be had.
@@ -486,7 +468,7 @@ void gaussian_mixture(RenderCtx& ctx, const Plane& in, const Plane& out, const s
             f.mode = k == 0 ? ACC_ZERO : ACC_PLANE;
             f.acc = &acc;
             f.weight = m.weight;
-            encode_blur(ctx, in, acc, m.sigma, f);
+            encode_fir(ctx, in, acc, a.t[0], f);
             continue;
         }
         // a run of components with a recursive channel, or one at a time when its planes are not to be had
@@ -775,7 +757,8 @@ Plane dir_couplers(RenderCtx& ctx, const Pipeline& p, const Plane& H, DevelopArg
             f.mode = ACC_ZERO;
             f.acc = &core;
             f.weight = fir[0].weight;
-            encode_blur(ctx, chi, core, fir[0].sigma, f);
+            const bool no_iir[3] = {false, false, false};  // one sigma for the three channels
+            encode_fir(ctx, chi, core, fir_taps(fir[0].sigma, no_iir), f);
         }
         if (!iir_mixture_mix(ctx, chi, iir, Vec3{0.0, 0.0, 0.0}, Vec3{1.0, 1.0, 1.0}))
             fail_internal("DIR diffusion: the recursive mixture was refused");
