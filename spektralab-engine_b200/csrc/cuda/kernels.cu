@@ -1324,6 +1324,18 @@ void ensure_smem(const void* kernel, int bytes) {
 }
 
 void set_launch_hook(LaunchHook* hook) { t_hook = hook; }
+uint32_t sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return uint32_t(n);
+}
+
 uint64_t launch_count() { return g_launches.load(); }
 
 void expose(const float* rgb, float* h, const float* patches, const ExposeArgs& a, cudaStream_t s) {
@@ -1520,7 +1532,7 @@ void source_copy(const float* raw, float* out, size_t pixels, uint32_t channels,
 
 void fill(void* p, size_t bytes, uint32_t v, cudaStream_t s) {
     Probe pr("fill", s);
-    k_fill<<<148 * 8, 256, 0, s>>>(static_cast<uint4*>(p), bytes / 16, v);
+    k_fill<<<sm_count() * 8, 256, 0, s>>>(static_cast<uint4*>(p), bytes / 16, v);
 }
 
 void sampler_poisson(const float* lam, float* out, uint32_t n, uint32_t stream, uint32_t seed, cudaStream_t s) {

@@ -32,6 +32,9 @@ struct Probe {
 // call. A new context (a host's own driver context, or one after a device reset) sets it afresh.
 void ensure_smem(const void* kernel, int bytes);
 
+// SMs of the current device (148 on a whole B200, fewer in a partition of one).
+uint32_t sm_count();
+
 // The driver's unique id of the current CUDA context; 0 when none is current or the driver cannot say.
 unsigned long long current_context_id();
 

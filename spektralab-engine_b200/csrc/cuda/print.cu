@@ -211,7 +211,7 @@ void print(const float* neg, float* rgb, const PrintArgs& a, cudaStream_t s) {
     const uint32_t threads = (a.n + 2 * kPairs - 1) / (2 * kPairs);
     // Fewer than two full CTAs per SM leave SMs idle or unevenly loaded: quarter-size ones spread such a print
     // (131 x 97: 0.0259 -> 0.0225 ms, 512 x 512: 0.0335 -> 0.0316; 1600 x 256 already 0.0427 -> 0.0482)
-    const uint32_t cta = threads < 2u * 148u * kPrintThreads ? kPrintThreads / 4 : kPrintThreads;
+    const uint32_t cta = threads < 2u * sm_count() * kPrintThreads ? kPrintThreads / 4 : kPrintThreads;
     Probe p("print", s);
     k_print<<<(threads + cta - 1) / cta, cta, 0, s>>>(neg, rgb, a);
 }

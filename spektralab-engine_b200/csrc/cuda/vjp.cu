@@ -537,7 +537,7 @@ void fir_pass_adjoint(const float* g_out, float* g_in, uint32_t w, uint32_t h, i
 void dot3(const float* x, const float* y, size_t pixels, double* acc, cudaStream_t s) {
     if (pixels == 0) return;
     Probe p("dot3", s);
-    k_dot3<<<148 * 4, kDotThreads, 0, s>>>(x, y, pixels, acc);
+    k_dot3<<<sm_count() * 4, kDotThreads, 0, s>>>(x, y, pixels, acc);
 }
 
 }  // namespace spkb::dev
