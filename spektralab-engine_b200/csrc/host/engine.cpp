@@ -2500,9 +2500,10 @@ SPK_API spk_status spk_render_vjp(spk_session* session, const char* tier, uint32
             });
         if (output && !grad_output)
             cuda_check(cudaMemcpyAsync(output, dy.ptr(), bytes, cudaMemcpyDeviceToHost, s.stream), "copy");
+        // the output is down before the gradient follows: an array given for both ends as the gradient
+        cuda_check(cudaStreamSynchronize(s.copy_stream), "render adjoint");
         if (grad_output)
             cuda_check(cudaMemcpyAsync(grad_input, dgx.ptr(), bytes, cudaMemcpyDeviceToHost, s.stream), "copy");
-        cuda_check(cudaStreamSynchronize(s.copy_stream), "render adjoint");
         cuda_check(cudaStreamSynchronize(s.stream), "render adjoint");
         cuda_check(cudaGetLastError(), "render adjoint");
         return SPK_OK;
