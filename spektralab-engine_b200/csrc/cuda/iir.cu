@@ -316,6 +316,14 @@ __device__ __forceinline__ void blur_lines(float* buf, int pitch, int nlines, in
 
 // 16-byte asynchronous copy global -> shared (both addresses 16-byte aligned), and the wait for all of
 // this thread's copies
+// blur_lines as a call: with registers for three CTAs an SM the inlined body spills into its loops (1600 x 200, eight
+// components 0.121 ms inlined, 0.089 called)
+template <int N>
+__device__ __noinline__ void blur_lines_call(float* buf, int pitch, int nlines, int n, int nseg, const IirPass<N>& q,
+                                             int comp, double* carry, bool seg_major) {
+    blur_lines(buf, pitch, nlines, n, nseg, q, comp, carry, seg_major);
+}
+
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
@@ -440,11 +448,9 @@ __device__ __forceinline__ void strip_sum(float* strip, int n, const IirSum& mix
 }
 
 // raw := mix_a raw + mix_b (the sum after the last component c), or the strip as it is (plain), in float4.
-// A thread steps down the rows kStoreBatch at a time, their reads issued before the first store (4K 0.239 ms at
-// one and two, 0.258 at four; 6000 x 4000 0.93, 0.88, 0.87).
-constexpr int kStoreBatch = 2;
-
-template <bool MULTI>
+// A thread steps down the rows BATCH at a time, their reads issued before the first store (4K 0.239 ms at one and
+// two, 0.258 at four; 6000 x 4000 0.93, 0.88, 0.87).
+template <bool MULTI, int BATCH>
 __device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, size_t pitch, int n, const IirSum& mix,
                                              int c, uint32_t tmem) {
     const int warp = int(threadIdx.x) >> 5, qd = int(threadIdx.x) % kQuads;
@@ -454,15 +460,15 @@ __device__ __forceinline__ void strip_to_raw(const float* strip, float* raw, siz
     int row = int(threadIdx.x) / kQuads;
     float* out = raw + size_t(row) * pitch + 4 * qd;
     const size_t step = size_t(kQuadRows) * pitch;
-    for (int q0 = 32 * warp; q0 < kQuads * n; q0 += kStoreBatch * kColThreads) {
-        float4 rw[kStoreBatch];
+    for (int q0 = 32 * warp; q0 < kQuads * n; q0 += BATCH * kColThreads) {
+        float4 rw[BATCH];
         if (!plain) {
 #pragma unroll
-            for (int u = 0; u < kStoreBatch; ++u)
+            for (int u = 0; u < BATCH; ++u)
                 if (row + u * kQuadRows < n) rw[u] = *reinterpret_cast<const float4*>(out + u * step);
         }
 #pragma unroll
-        for (int u = 0; u < kStoreBatch; ++u) {
+        for (int u = 0; u < BATCH; ++u) {
             if (q0 + u * kColThreads >= kQuads * n) break;
             const int r = min(row, n - 1);
             float4 v = *reinterpret_cast<const float4*>(strip + size_t(r) * kColLines + 4 * qd);
@@ -506,11 +512,11 @@ __device__ __forceinline__ void strip_to_raw_scalar(const float* strip, float* r
     }
 }
 
-// MULTI: more than one component, the sum in tensor memory. Registers for two strips per SM (what shared
-// memory holds at 4K): held to three or four, even short frames ran slower (1024 x 1024, one component: 0.030 ms
-// at two, 0.035 and 0.038).
-template <bool MULTI, int N>
-__global__ void __launch_bounds__(kColThreads, 2) k_iir_cols(float* raw, const __grid_constant__ IirPlanes hs, uint32_t w, uint32_t h,
+// MULTI: more than one component, the sum in tensor memory. CTAS: the strips per SM that the registers allow. Two
+// (what shared memory holds at 4K) are faster each; a strip of a short frame is latency from barrier to
+// barrier, and where there are more than two for every SM three at a time are faster together (three_strips).
+template <bool MULTI, int N, int CTAS>
+__global__ void __launch_bounds__(kColThreads, CTAS) k_iir_cols(float* raw, const __grid_constant__ IirPlanes hs, uint32_t w, uint32_t h,
                                                           const __grid_constant__ IirSum mix,
                                                           const __grid_constant__ IirPass<N> pass,
                                                           const __grid_constant__ IirColMaps maps) {
@@ -586,11 +592,12 @@ __global__ void __launch_bounds__(kColThreads, 2) k_iir_cols(float* raw, const _
             }
         }
         __syncthreads();
-        blur_lines(strip, kColLines, kColLines, n, kSegCols, pass, c, carry, false);
+        if (CTAS == 2) blur_lines(strip, kColLines, kColLines, n, kSegCols, pass, c, carry, false);
+        else blur_lines_call(strip, kColLines, kColLines, n, kSegCols, pass, c, carry, false);
         if (MULTI && c + 1 < int(mix.ncomp)) {
             strip_sum<MULTI>(strip, n, mix, c, tmem, false);
         } else if (raw_vec) {
-            strip_to_raw<MULTI>(strip, raw + off, raw_pitch, n, mix, c, tmem);
+            strip_to_raw<MULTI, CTAS == 2 ? 2 : 1>(strip, raw + off, raw_pitch, n, mix, c, tmem);
         } else {
             if (mix.plain == 0) {
                 strip_sum<MULTI>(strip, n, mix, c, tmem, true);
@@ -723,13 +730,23 @@ bool col_maps(IirColMaps& maps, const IirPlanes& planes, uint32_t ncomp, uint32_
     return true;
 }
 
+// Whether the column pass runs three strips an SM: more strips than two for every SM, in frames short enough.
+// Column pass with two and three, 1, 2 and 3 components: 1600 x 200 0.025 / 0.021, 0.040 / 0.031, 0.056 / 0.042 ms;
+// 4096 x 64 0.027 / 0.027, 0.048 / 0.044, 0.064 / 0.060; 1600 x 600 0.033 / 0.029, 0.052 / 0.046, 0.072 / 0.058;
+// 1600 x 1067 0.044 / 0.044, 0.070 / 0.064, 0.095 / 0.087; 3552 x 900 one component 9 % slower with three, 3552 x 1300
+// 19, 9 and 2 % slower. At 1100 rows three strips take 186 KB of shared memory and 384 columns of tensor memory.
+bool three_strips(uint32_t w, uint32_t h, uint32_t ncomp) {
+    return (w + kColPixels - 1) / kColPixels > 2 * sm_count() && h <= (ncomp > 1 ? 1100u : 500u);
+}
+
 template <int N>
 void launch_passes(const float* src, float* raw, const IirPlanes& planes, uint32_t w, uint32_t h, const IirMixture& m,
                    const IirColMaps& maps, cudaStream_t s) {
     const size_t sr = iir_rows_smem(m.pitch), sc = iir_cols_smem(h);
     constexpr bool kMulti = N > 1;
     ensure_smem(reinterpret_cast<const void*>(k_iir_rows<N>), int(sr));
-    ensure_smem(reinterpret_cast<const void*>(k_iir_cols<kMulti, N>), int(sc));
+    const auto cols = three_strips(w, h, m.ncomp) ? k_iir_cols<kMulti, N, 3> : k_iir_cols<kMulti, N, 2>;
+    ensure_smem(reinterpret_cast<const void*>(cols), int(sc));
     {
         Probe p("iir_rows", s);
         k_iir_rows<N><<<h, kRowThreads, sr, s>>>(src, planes, w, h, m, IirPass<N>(m.rows, m.ncomp));
@@ -737,7 +754,7 @@ void launch_passes(const float* src, float* raw, const IirPlanes& planes, uint32
     {
         Probe p("iir_cols", s);
         const uint32_t g = (w + kColPixels - 1) / kColPixels;
-        k_iir_cols<kMulti, N><<<g, kColThreads, sc, s>>>(raw, planes, w, h, m, IirPass<N>(m.cols, m.ncomp), maps);
+        cols<<<g, kColThreads, sc, s>>>(raw, planes, w, h, m, IirPass<N>(m.cols, m.ncomp), maps);
     }
 }
 }  // namespace
