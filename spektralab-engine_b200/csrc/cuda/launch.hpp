@@ -99,7 +99,8 @@ void develop_rows(const float* exposure, float* out, const DevelopArgs& a, uint3
 void develop_prepare(cudaStream_t s);
 
 // negative density -> linear output RGB (enlarger, gain, paper, scan, XYZ -> RGB, CAM16 gamut).
-void print(const float* neg, float* rgb, const PrintArgs& a, cudaStream_t s);
+// beside: how many prints of about this size the caller runs at the same time, this one counted.
+void print(const float* neg, float* rgb, const PrintArgs& a, cudaStream_t s, uint32_t beside = 1);
 
 // The print stage with the spectral integrals in the given SpectralMode (print_tc.cu): host_tab the
 // tables on the host (their binary32 part goes into the kernel's parameters), tab the same in device

@@ -206,12 +206,16 @@ __global__ void __launch_bounds__(kPrintThreads) k_print_batch_shared(const Batc
 
 }  // namespace
 
-void print(const float* neg, float* rgb, const PrintArgs& a, cudaStream_t s) {
+void print(const float* neg, float* rgb, const PrintArgs& a, cudaStream_t s, uint32_t beside) {
     if (a.n == 0) return;
     const uint32_t threads = (a.n + 2 * kPairs - 1) / (2 * kPairs);
     // Fewer than two full CTAs per SM leave SMs idle or unevenly loaded: quarter-size ones spread such a print
-    // (131 x 97: 0.0259 -> 0.0225 ms, 512 x 512: 0.0335 -> 0.0316; 1600 x 256 already 0.0427 -> 0.0482)
-    const uint32_t cta = threads < 2u * sm_count() * kPrintThreads ? kPrintThreads / 4 : kPrintThreads;
+    // (131 x 97: 0.0259 -> 0.0225 ms, 512 x 512: 0.0335 -> 0.0316; 1600 x 256 already 0.0427 -> 0.0482). Prints of
+    // other frames at the same time fill the SMs too, and full CTAs then share more of their instructions
+    // (a batch of eight 512 x 512 on four streams 0.622 ms with quarter-size CTAs, 0.597 with full ones; on
+    // sixteen 0.713 and 0.665; of 24 131 x 97 on four 0.698 and 0.711).
+    const bool quarter = uint64_t(threads) * beside < 2u * sm_count() * kPrintThreads;
+    const uint32_t cta = quarter ? kPrintThreads / 4 : kPrintThreads;
     Probe p("print", s);
     k_print<<<(threads + cta - 1) / cta, cta, 0, s>>>(neg, rgb, a);
 }

@@ -903,7 +903,7 @@ void run_plan(Engine& e, const std::string& plan, const std::string& shape, std:
                     BatchFrame& f = fr[slots[j]];
                     cudaStream_t ws = e.workers[j % K];
                     cuda_check(cudaStreamWaitEvent(ws, f.ready, cudaEventWaitExternal), "frame ready");
-                    dev::print(f.neg, f.rgb.data(), f.pa, ws);
+                    dev::print(f.neg, f.rgb.data(), f.pa, ws, uint32_t(K));
                     dev::scan_encode(f.rgb.data(), f.img->dev, f.rgb.w, f.rgb.h, f.sa, ws);
                     cuda_check(cudaMemcpyAsync(f.img->host, f.img->dev, f.img->bytes, cudaMemcpyDeviceToHost, ws),
                                "result copy");
