@@ -190,7 +190,8 @@ __device__ __forceinline__ void scan_tile(const ScanArgs& a, const float* __rest
         const float* bc = A + (i + r2) * BC + 3 * (lane + r2);
         float v0 = bc[0], v1 = bc[1], v2 = bc[2];
         if (e.unsharp) {
-            const float* vr = B + i * BC + 3 * lane;
+            // a radius of 0 (a mask of a small tier of a large frame): the one tap on the tile itself, no pass before
+            const float* vr = r2 > 0 ? B + i * BC + 3 * lane : bc;
             float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
 #pragma unroll
             for (int k = 0; k <= 2 * r2; ++k) {
