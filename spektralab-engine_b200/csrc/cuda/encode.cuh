@@ -19,9 +19,12 @@ __device__ __forceinline__ void mat_apply(const float* m, float x, float y, floa
 }
 
 // x^y for x >= 0 (NaN for x < 0, 0 for x = 0, y > 0) as 2^(y log2 x) on the special-function unit
-// (PTX lg2.approx and ex2.approx, subnormals to zero): relative error within about 2^-22 (1 + |y log2 x|),
-// against 2 ulp for powf. Every use feeds a 16-bit output, whose 1 LSB is 2^-16 of full scale; the
-// render tests hold the output to the binary64 oracle and to the reference's precise-math build.
+// (PTX lg2.approx and ex2.approx): relative error within about 2^-22 (1 + |y log2 x|), against 2 ulp for
+// powf. Every use feeds a 16-bit output, whose 1 LSB is 2^-16 of full scale; the render tests hold the
+// output to the binary64 oracle and to the reference's precise-math build.
+// The .ftz forms take subnormal operands (of either sign) and results for 0: one instruction each, where the
+// others scale around it. Of the transfer functions only the Adobe RGB one is asked for so small a value, and
+// its result, below 2^-57, is code 0 as 0 and NaN are; the print's uses are further from it (print_common.cuh).
 __device__ __forceinline__ float powm(float x, float y) {
     float l, r;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x));

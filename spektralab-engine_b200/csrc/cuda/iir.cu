@@ -29,7 +29,9 @@
 //             With three components at 6000 x 4000 the loads take 0.29 ms, raw 0.28, the recurrences the rest
 //             (one strip of twelve warps per SM; the 32-to-64-bit conversions' unit is the busiest there).
 //             Loading and converting eight samples ahead of their chain made the recurrences slower (0.88 ->
-//             1.09 ms; rows at 4K 0.150 -> 0.187): the unrolled loop already overlaps them. Its waits are bounded: one that gives up counts
+//             1.09 ms; rows at 4K 0.150 -> 0.187): the unrolled loop already overlaps them. Short frames with
+//             many strips run three strips an SM instead of two (three_strips).
+//             Its waits are bounded: one that gives up counts
 //             itself (g_iir_gave_up), waits again under the full limit for the copies in flight, and if
 //             even they never land the CTA loads this and every later strip with plain copies.
 #include <cuda.h>

@@ -56,8 +56,9 @@ __device__ __forceinline__ float lg2_approx(float x) {
     return y;
 }
 // The approximate operations take their .ftz forms, one special-function instruction each: the others
-// scale subnormal operands and results around it, and no value here that is not zero is below 1e-30 (the
-// sums carry kTiny, the gamut stage works on percentages). Same results on normal numbers.
+// scale subnormal operands and results around it. Same results on normal numbers, and a subnormal here changes
+// nothing: the sums carry kTiny, post_adapt's power is added to 27.13, and the gamut stage's small values are
+// differences of its results (0.1 and above, so zero or 1e-9 and more) or their squares.
 // a / b with PTX div.approx (2 ulp for |b| in [2^-126, 2^126]); a / 0 = +-inf, 0 / 0 = NaN
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float fsqrt(float x) {

@@ -58,12 +58,12 @@ private:
     std::shared_ptr<PoolState> s_;
 };
 
-// The device memory pool behind every Pool: keep all freed memory cached (release threshold max).
 // Whether kernels on `device` may read the caller's `bytes` at p where they lie: 16-byte aligned device memory of
 // that device, all of it within one allocation. Anything else is left to a copy, which takes any alignment and
 // other devices' memory and whose driver checks the range.
 bool readable_in_place(const void* p, size_t bytes, int device);
 
+// The device memory pool behind every Pool: keep all freed memory cached (release threshold max).
 void configure_device_pool(int device);
 size_t device_pool_trim(int device);          // returns the cached bytes released to the driver
 size_t device_pool_reserved(int device);
